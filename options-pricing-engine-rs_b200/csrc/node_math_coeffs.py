@@ -14,7 +14,9 @@ log v = k ln 2 + 2 atanh(s), s = (m - 1)/(m + 1), |s| <= 3 - 2 sqrt 2, and
 interpolates (2 atanh(s) - 2 s)/(s w) at the 7 Chebyshev nodes of
 [0, (3 - 2 sqrt 2)^2]: 4.5e-18 relative error on log m.
 
-Both are far below the 1.1e-16 rounding unit; the evaluation in double
+log_ratio takes the same R over |s| <= 0.2016 at degree 7 (8 nodes): 5.8e-19.
+
+All are far below the 1.1e-16 rounding unit; the evaluation in double
 precision then adds a few ulps (checked against CUDA's functions on the
 device by ope_selftest_atan2 / ope_selftest_log and in numpy by
 tests/test_node_math_cpu.py).
@@ -27,6 +29,8 @@ import mpmath as mp
 mp.mp.dps = 60
 ATAN_DEG = 10
 LOG_DEG = 6
+LOG_RATIO_DEG = 7
+LOG_RATIO_S = mp.mpf("0.2016")
 
 
 def _chebyshev_interpolant(fn, hi, deg):
@@ -64,6 +68,12 @@ def log_coefficients(deg=LOG_DEG):
     return _chebyshev_interpolant(_log_r, wmax, deg), wmax
 
 
+def log_ratio_coefficients(deg=LOG_RATIO_DEG):
+    """R(w) of log_ratio, lowest degree first, and the interval end."""
+    wmax = LOG_RATIO_S ** 2
+    return _chebyshev_interpolant(_log_r, wmax, deg), wmax
+
+
 def _poly(c, x):
     return sum(c[j] * x ** j for j in range(len(c)))
 
@@ -80,7 +90,8 @@ def log_error(c, wmax, samples=2000):
 
 if __name__ == "__main__":
     for name, (c, hi), err in (("atan2_node P(s)", atan_coefficients(), atan_error),
-                               ("log_node R(w)", log_coefficients(), log_error)):
+                               ("log_node R(w)", log_coefficients(), log_error),
+                               ("log_ratio R(w)", log_ratio_coefficients(), log_error)):
         print(name)
         for j in reversed(range(len(c))):
             print(f"    {float(c[j])!r},  // ^{j}")

@@ -1,0 +1,39 @@
+"""The node evaluation where its branches turn: correlations beyond +-1 (the
+square root's argument crosses into the left half plane), a vol-of-vol near 0,
+kappa below rho sigma (the P1 normaliser degenerates), jumps switched off and
+one-sided, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from ope_b200 import workloads as W
+
+PARAMS = [(0.04, 1.5, 0.04, 0.5, 1.0), (0.04, 1.5, 0.04, 0.5, -1.0), (0.09, 0.5, 0.06, 1e-3, -0.4),
+          (0.04, 0.1, 0.04, 0.9, 0.5), (0.04, 4.0, 0.09, 0.3, 0.0)]
+JUMPS = [None, (0.0, 0.0, 0.1), (1.2, -0.3, 0.05), (0.4, 0.1, 0.6)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("jump", JUMPS)
+@pytest.mark.parametrize("heston", PARAMS)
+def test_prices_at_the_branches_of_the_node_evaluation(ope, oracle, heston, jump):
+    """At the parity bar, 1e-9 S."""
+    con = W.c1().contracts.copy()
+    con["expiry"] *= np.where(np.arange(con.size) % 3 == 0, 0.02, 1.0)
+    par = np.array(heston + (jump or ()))
+    got = (ope.batch_heston if jump is None else ope.batch_bates)(con, par, tol=1e-10)
+    ref = oracle.batch_price(con, par[None, :], jump is not None, 1e-10)
+    assert np.max(np.abs(got - ref)) <= 1e-9 * 100.0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", [0, 1])
+@pytest.mark.parametrize("rho", [1.2, -1.3])
+def test_nodes_beyond_correlation_one(ope, oracle, rho, which):
+    """The integrals diverge there, so the 30 nodes of the first bisection are
+    compared: 1e-11 of the largest, the bar of the corner traces."""
+    con, par = W.c1().contracts[37:38], np.array((0.04, 1.5, 0.04, 0.5, rho))
+    got, _ = ope.trace_integral(ope.MODEL_HESTON, con, par, which, tol=1e-10)
+    ref, _ = oracle.trace_integral(con, par, False, which, 1e-10)
+    a, b = got[0, 9:39], ref[0, 9:39]
+    assert np.array_equal(np.isfinite(a), np.isfinite(b))
+    assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(b))
