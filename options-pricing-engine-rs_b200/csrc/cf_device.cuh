@@ -164,6 +164,146 @@ __device__ __forceinline__ double log_ratio(double a, double b, double& ia) {
     return fma(kd, 0.6931471805599453, fma(kd, 2.3190468138462996e-17, fma(s * w, r, 2.0 * s)));
 }
 
+// Tables of the node evaluation's own exponential and sine/cosine: 2^(j/64),
+// and (cos, sin) of j pi/32, correctly rounded.  Read by index through L1.
+static __device__ const double g_exp2_tab[64] = {
+    1.0, 1.0108892860517005, 1.0218971486541166, 1.0330248790212284,
+    1.0442737824274138, 1.0556451783605572, 1.0671404006768237, 1.0787607977571199,
+    1.0905077326652577, 1.102382583307841, 1.1143867425958924, 1.1265216186082418,
+    1.1387886347566916, 1.1511892299529827, 1.1637248587775775, 1.1763969916502812,
+    1.189207115002721, 1.202156731452703, 1.215247359980469, 1.22848053610687,
+    1.241857812073484, 1.255380757024691, 1.2690509571917332, 1.2828700160787783,
+    1.2968395546510096, 1.3109612115247644, 1.3252366431597413, 1.339667524053303,
+    1.3542555469368927, 1.3690024229745905, 1.383909881963832, 1.3989796725383112,
+    1.4142135623730951, 1.42961333839197, 1.4451808069770467, 1.460917794180647,
+    1.4768261459394993, 1.4929077282912648, 1.5091644275934228, 1.5255981507445384,
+    1.5422108254079407, 1.559004400237837, 1.5759808451078865, 1.593142151342267,
+    1.6104903319492543, 1.6280274218573478, 1.645755478153965, 1.6636765803267364,
+    1.681792830507429, 1.7001063537185235, 1.718619298122478, 1.7373338352737062,
+    1.7562521603732995, 1.7753764925265212, 1.7947090750031072, 1.8142521755003989,
+    1.8340080864093424, 1.8539791250833855, 1.8741676341103, 1.8945759815869656,
+    1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951};
+static __device__ const double2 g_cis_tab[64] = {
+    {1.0, 0.0}, {0.9951847266721969, 0.0980171403295606},
+    {0.9807852804032304, 0.19509032201612828}, {0.9569403357322088, 0.2902846772544624},
+    {0.9238795325112867, 0.3826834323650898}, {0.881921264348355, 0.47139673682599764},
+    {0.8314696123025452, 0.5555702330196022}, {0.773010453362737, 0.6343932841636455},
+    {0.7071067811865476, 0.7071067811865476}, {0.6343932841636455, 0.773010453362737},
+    {0.5555702330196022, 0.8314696123025452}, {0.47139673682599764, 0.881921264348355},
+    {0.3826834323650898, 0.9238795325112867}, {0.2902846772544624, 0.9569403357322088},
+    {0.19509032201612828, 0.9807852804032304}, {0.0980171403295606, 0.9951847266721969},
+    {0.0, 1.0}, {-0.0980171403295606, 0.9951847266721969},
+    {-0.19509032201612828, 0.9807852804032304}, {-0.2902846772544624, 0.9569403357322088},
+    {-0.3826834323650898, 0.9238795325112867}, {-0.47139673682599764, 0.881921264348355},
+    {-0.5555702330196022, 0.8314696123025452}, {-0.6343932841636455, 0.773010453362737},
+    {-0.7071067811865476, 0.7071067811865476}, {-0.773010453362737, 0.6343932841636455},
+    {-0.8314696123025452, 0.5555702330196022}, {-0.881921264348355, 0.47139673682599764},
+    {-0.9238795325112867, 0.3826834323650898}, {-0.9569403357322088, 0.2902846772544624},
+    {-0.9807852804032304, 0.19509032201612828}, {-0.9951847266721969, 0.0980171403295606},
+    {-1.0, 0.0}, {-0.9951847266721969, -0.0980171403295606},
+    {-0.9807852804032304, -0.19509032201612828}, {-0.9569403357322088, -0.2902846772544624},
+    {-0.9238795325112867, -0.3826834323650898}, {-0.881921264348355, -0.47139673682599764},
+    {-0.8314696123025452, -0.5555702330196022}, {-0.773010453362737, -0.6343932841636455},
+    {-0.7071067811865476, -0.7071067811865476}, {-0.6343932841636455, -0.773010453362737},
+    {-0.5555702330196022, -0.8314696123025452}, {-0.47139673682599764, -0.881921264348355},
+    {-0.3826834323650898, -0.9238795325112867}, {-0.2902846772544624, -0.9569403357322088},
+    {-0.19509032201612828, -0.9807852804032304}, {-0.0980171403295606, -0.9951847266721969},
+    {0.0, -1.0}, {0.0980171403295606, -0.9951847266721969},
+    {0.19509032201612828, -0.9807852804032304}, {0.2902846772544624, -0.9569403357322088},
+    {0.3826834323650898, -0.9238795325112867}, {0.47139673682599764, -0.881921264348355},
+    {0.5555702330196022, -0.8314696123025452}, {0.6343932841636455, -0.773010453362737},
+    {0.7071067811865476, -0.7071067811865476}, {0.773010453362737, -0.6343932841636455},
+    {0.8314696123025452, -0.5555702330196022}, {0.881921264348355, -0.47139673682599764},
+    {0.9238795325112867, -0.3826834323650898}, {0.9569403357322088, -0.2902846772544624},
+    {0.9807852804032304, -0.19509032201612828}, {0.9951847266721969, -0.0980171403295606}};
+
+// Adding 1.5 2^52 rounds a double of magnitude below 2^51 to the nearest
+// integer, left in the low word of the sum.
+constexpr double kRound = 6755399441055744.0;
+
+// The phases exp_node, cis_node and sin_node take must lie below 2^45 in
+// magnitude (node_range: the largest of them, as the high word without its
+// sign; kRangeEnd: 2^45).  Beyond, where a phase's own ulp passes 2^-8, and
+// for non-finite phases, the node takes node_slow.
+constexpr unsigned kRangeEnd = 2u * 0x42C00000u;
+__device__ __forceinline__ unsigned node_range(double x) { return 2u * (unsigned)__double2hiint(x); }
+
+// e^x, branch-free (table-driven after Tang, ACM TOMS 15, 1989): x = k ln2/64
+// + r, |r| <= ln2/128, e^x = 2^(k/64) (1 + r + r^2 P(r)), P the degree-3
+// Chebyshev interpolant of node_math_coeffs.py (4e-18 absolute), ln2/64 split
+// into a double and its remainder.  x below -708 is taken as -708 (3e-308)
+// and above 710 as 710 (infinity or NaN); NaN stays NaN.  In place of CUDA's
+// exp on the 262k-contract Bates batch: 11.05 -> 10.61 ms (after cis_node and
+// sin_node); a degree-11 polynomial without the table: 10.96 ms.
+__device__ __forceinline__ double exp_node(double x) {
+    int hx = __double2hiint(x);
+    if (x < -708.0) hx = 0xC0862000;  // the high word of -708
+    hx = min(hx, 0x40863000);         // of 710 (a negative x is a negative int)
+    x = __hiloint2double(hx, __double2loint(x));
+    const double t = fma(x, 92.33248261689366, kRound);  // 64/ln2
+    const int k = __double2loint(t);
+    const double kd = __dsub_rn(t, kRound);
+    const double tab = __ldg(g_exp2_tab + (k & 63));
+    double r = fma(kd, -0.010830424696249145, x);
+    r = fma(kd, -3.623510646634843e-19, r);
+    double q = 0.008333339151693497;
+    q = fma(q, r, 0.04166670739519196);
+    q = fma(q, r, 0.16666666666664534);
+    q = fma(q, r, 0.49999999999985073);
+    q = fma(q, __dmul_rn(r, r), r);
+    const double sc = __hiloint2double(__double2hiint(tab) + ((k >> 6) << 20), __double2loint(tab));
+    return fma(sc, q, sc);
+}
+
+// m e^{ix}, branch-free: x = k pi/32 + r, |r| <= pi/64, pi/32 split into a
+// double and its remainder, sin r and cos r - 1 from the Chebyshev
+// interpolants of node_math_coeffs.py (1.4e-19 and 2.6e-17 absolute), then
+// the angle sum with the table's (cos, sin) of k pi/32.  Error a rounding or
+// two of 1 per component before the product with m.  In place of CUDA's
+// sincos, with sin_node: 11.98 -> 11.05 ms on the same batch; reduced by pi
+// with two longer polynomials and no table: 11.46 ms.
+__device__ __forceinline__ void cis_node(double m, double x, double& re, double& im) {
+    const double t = fma(x, 10.185916357881302, kRound);  // 32/pi
+    const int k = __double2loint(t);
+    const double kd = __dsub_rn(t, kRound);
+    const double2 cs = __ldg(g_cis_tab + (k & 63));
+    double r = fma(kd, -0.09817477042468103, x);
+    r = fma(kd, -3.827021247335479e-18, r);
+    const double w = __dmul_rn(r, r);
+    double a = fma(-0.00019840273845896154, w, 0.008333333324333688);
+    a = fma(a, w, -0.16666666666666546);
+    const double sr = fma(__dmul_rn(a, w), r, r);  // sin r
+    double b = fma(-0.001388799249796147, w, 0.041666666585670434);
+    b = fma(b, w, -0.4999999999999892);
+    const double cm = __dmul_rn(b, w);  // cos r - 1
+    re = __dmul_rn(m, fma(-cs.y, sr, fma(cs.x, cm, cs.x)));
+    im = __dmul_rn(m, fma(cs.x, sr, fma(cs.y, cm, cs.y)));
+}
+
+// sin(x + a) w, branch-free, x taken as exact and reduced before a is added:
+// k the integer nearest (x + a)/pi, r = (x - k pi) + a, |r| <= pi/2 (the first
+// subtraction is one FMA, so it rounds at the size of a, not of x), sin r =
+// r + r s Q(s), s = r^2, Q the degree-7 Chebyshev interpolant (1.3e-18
+// absolute), the sign (-1)^k put on w.
+__device__ __forceinline__ double sin_node(double x, double a, double w) {
+    const double t = fma(__dadd_rn(x, a), 0.3183098861837907, kRound);  // 1/pi
+    const int k = __double2loint(t);
+    const double kd = __dsub_rn(t, kRound);
+    double r = fma(kd, -3.141592653589793, x);
+    r = __dadd_rn(fma(kd, -1.2246467991473532e-16, r), a);
+    const double s = __dmul_rn(r, r);
+    double q = 2.7314447669863995e-15;
+    q = fma(q, s, -7.643970296798572e-13);
+    q = fma(q, s, 1.6058977312464087e-10);
+    q = fma(q, s, -2.5052107616996182e-08);
+    q = fma(q, s, 2.7557319219163234e-06);
+    q = fma(q, s, -0.00019841269841254974);
+    q = fma(q, s, 0.008333333333333316);
+    q = fma(q, s, -0.16666666666666666);
+    const double sw = __hiloint2double(__double2hiint(w) ^ (k << 31), __double2loint(w));
+    return __dmul_rn(fma(__dmul_rn(q, s), r, r), sw);
+}
+
 // Error-free transformations (Knuth's TwoSum, Dekker's Fast2Sum, the FMA
 // product residual) and double-double arithmetic, for log_cr below.
 __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e) {
@@ -310,7 +450,7 @@ __device__ __forceinline__ void csqrt_node(double zr, double zi, double& dre, do
 // own, and a node takes one complex reciprocal (of N) where the literal
 // sequence takes four.
 struct CfConsts {
-    double xr, rs, zr0, zr2, zi1, kts, ktst, nv0, sgn, t, rtl, z0re, z0im;
+    double xr, rs, zr0, zr2, zi1, kts, ktst, kts2, nv0, sgn, t, rtl, z0re, z0im;
     double jr0, hs2, jmu, lt, jre0;
     // raw values kept for the adjoint chain
     double kappa, phi_im, sig2, v0s, rt, x, lnm_re, lnm_im, mu_j, comp;
@@ -369,6 +509,7 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
     C.zr2 = C.sig2 * ((1.0 - rho) * (1.0 + rho));
     C.zi1 = fma(-2.0 * C.xr, C.rs, C.sig2 * C.sgn);
     C.ktst = C.kts * t;
+    C.kts2 = 2.0 * C.kts;
     C.nv0 = -v0;
     double lt = 0.0, mu_j = 0.0, hs2 = 0.0, comp = 0.0;
     if (bates) {
@@ -450,60 +591,99 @@ __device__ __forceinline__ double node_u_of(double tn) {
     return u;
 }
 
+// FAST: branch-free, with the functions above; `range` receives what decides
+// whether they applied (compare with kRangeEnd): the phases of e^{-dT} and of
+// the jump factor, and the sign of Re z (negative only for |rho| > 1).  Not
+// FAST: CUDA's functions and the square root's other branch.
+//
 // What bounds it: issue slots.  The form without g (CfConsts above), the
 // merged reciprocals and the third-order refinements took the 1M-contract
 // Bates batch from 51.2 to 47.5 ms (262k contracts: 12.99 to 12.03 ms; the
-// same contracts under Heston 11.45 to 10.52 ms).
-template <bool BATES>
-__device__ __forceinline__ NodeCf node_cf(const CfConsts& C, double tn) {
+// same contracts under Heston 11.45 to 10.52 ms); the own exponential, sine
+// and cosine, with their range tests gathered into one branch per node, took
+// the 262k batches on to 10.17 and 8.95 ms (865 to 662 instructions per warp
+// step, 317 to 252 of them FP64).
+template <bool BATES, bool FAST>
+__device__ __forceinline__ NodeCf node_eval(const CfConsts& C, double tn, unsigned& range) {
     double u, itt;  // (1 - t) / t and 1 / ((1 - t) t)
     node_geom(tn, u, itt);
-    const double u2 = u * u;
+    const double u2 = __dmul_rn(u, u);
     // xi = (xr, xi_) ; z = xi^2 + sigma^2 phi(phi+i) = (xr^2 + zr2 u^2, zi1 u)
-    const double xi_ = -C.rs * u;
-    const double zr = fma(C.zr2, u2, C.zr0), zi = C.zi1 * u;
+    const double xi_ = __dmul_rn(-C.rs, u);
+    const double zr = fma(C.zr2, u2, C.zr0), zi = __dmul_rn(C.zi1, u);
     // d = sqrt z: Re d = sqrt((|z| + Re z) / 2), Im d = Im z / (2 Re d)
-    const double zz = fma(zr, zr, zi * zi);
-    const double hr = 0.5 * zz * rsqrt_nr(zz);  // |z| / 2
-    const double s2 = fma(0.5, fabs(zr), hr);
+    const double zz = fma(zr, zr, __dmul_rn(zi, zi));
+    const double hr = __dmul_rn(__dmul_rn(0.5, zz), rsqrt_nr(zz));  // |z| / 2
+    const double s2 = fma(0.5, FAST ? zr : fabs(zr), hr);
     const double iw = rsqrt_nr(s2);
-    double dre = s2 * iw, dim = (0.5 * zi) * iw;
-    if (C.zr2 < 0.0 && zr < 0.0) {  // |rho| > 1: Re z may be negative
+    double dre = __dmul_rn(s2, iw), dim = __dmul_rn(__dmul_rn(0.5, zi), iw);
+    if (!FAST && zr < 0.0) {
         const double w = dre;
         dre = fabs(dim);
         dim = copysign(w, zi);
     }
-    const double mr = C.xr - dre, mi = xi_ - dim;  // m = xi - d
-    const double pr = C.xr + dre, pi = xi_ + dim;  // p = xi + d
+    const double mr = __dsub_rn(C.xr, dre), mi = __dsub_rn(xi_, dim);  // m = xi - d
+    const double pr = __dadd_rn(C.xr, dre), pi = __dadd_rn(xi_, dim);  // p = xi + d
     // e = exp(-d T)
-    double sn, cs;
-    sincos(-dim * C.t, &sn, &cs);
-    const double em = exp(-dre * C.t);
-    const double er = em * cs, ei = em * sn;
+    const double th = __dmul_rn(-dim, C.t), et = __dmul_rn(-dre, C.t);
+    double er, ei;
+    if (FAST) {
+        range = max(node_range(th), (unsigned)__double2hiint(zr));  // Re z < 0: above kRangeEnd
+        cis_node(exp_node(et), th, er, ei);
+    } else {
+        sincos(th, &ei, &er);
+        const double em = exp(et);
+        er = __dmul_rn(em, er);
+        ei = __dmul_rn(em, ei);
+    }
     // N = p - m e
     const double nr = fma(mi, ei, fma(-mr, er, pr));
     const double ni = fma(-mr, ei, fma(-mi, er, pi));
-    const double nn = fma(nr, nr, ni * ni);
+    const double nn = fma(nr, nr, __dmul_rn(ni, ni));
     // Log A, A = N / (2 d): |A|^2 = nn / (4 |z|), arg A = arg(N conj(d))
     double ia;
-    const double la = log_ratio(nn, 8.0 * hr, ia);
-    const double li = atan2_node(fma(ni, dre, -nr * dim), fma(nr, dre, ni * dim));
+    const double la = log_ratio(nn, __dmul_rn(8.0, hr), ia);
+    const double li = atan2_node(fma(ni, dre, __dmul_rn(-nr, dim)), fma(nr, dre, __dmul_rn(ni, dim)));
     // D = -v0 phi(phi+i) (1 - e) / N, phi(phi+i) = u (u + i sgn)
-    const double omr = 1.0 - er;
-    const double qr = fma(omr, nr, -ei * ni), qi = -fma(ei, nr, omr * ni);
-    const double s = (C.nv0 * u) * ia;
-    const double Dr = fma(u, qr, -C.sgn * qi), Di = fma(u, qi, C.sgn * qr);
+    const double omr = __dsub_rn(1.0, er);
+    const double qr = fma(omr, nr, __dmul_rn(-ei, ni)), qi = fma(-ei, nr, __dmul_rn(-omr, ni));
+    const double s = __dmul_rn(__dmul_rn(C.nv0, u), ia);
+    const double Dr = fma(u, qr, __dmul_rn(-C.sgn, qi)), Di = fma(u, qi, __dmul_rn(C.sgn, qr));
     // Re, Im Z = kts ((xi - d) T - 2 Log A) + D + z0 + i (r T u)
     double zre = fma(C.ktst, mr, fma(-C.kts, la, fma(s, Dr, C.z0re)));
-    double zim = fma(C.ktst, mi, fma(-2.0 * C.kts, li, fma(s, Di, fma(C.rtl, u, C.z0im))));
+    double zim = fma(C.ktst, mi, fma(-C.kts2, li, fma(s, Di, fma(C.rtl, u, C.z0im))));
     if (BATES) {
-        double js, jc;
-        sincos(C.jmu * u, &js, &jc);
-        const double je = C.lt * exp(fma(-C.hs2, u2, C.jr0));
-        zre += fma(je, jc, C.jre0);
-        zim = fma(je, js, zim);
+        const double tj = __dmul_rn(C.jmu, u), ej = fma(-C.hs2, u2, C.jr0);
+        double jr, ji;
+        if (FAST) {
+            range = max(range, node_range(tj));
+            cis_node(__dmul_rn(C.lt, exp_node(ej)), tj, jr, ji);
+        } else {
+            sincos(tj, &ji, &jr);
+            const double je = __dmul_rn(C.lt, exp(ej));
+            jr = __dmul_rn(je, jr);
+            ji = __dmul_rn(je, ji);
+        }
+        zre = __dadd_rn(zre, __dadd_rn(jr, C.jre0));
+        zim = __dadd_rn(zim, ji);
     }
-    return NodeCf{exp(zre), zim, u, itt};
+    return NodeCf{FAST ? exp_node(zre) : exp(zre), zim, u, itt};
+}
+
+// The rare nodes out of the fast functions' range (internal linkage: within
+// the calling kernel's register budget).
+template <bool BATES>
+static __device__ __noinline__ NodeCf node_slow(const CfConsts& C, double tn) {
+    unsigned range;
+    return node_eval<BATES, false>(C, tn, range);
+}
+
+template <bool BATES>
+__device__ __forceinline__ NodeCf node_cf(const CfConsts& C, double tn) {
+    unsigned range;
+    NodeCf n = node_eval<BATES, true>(C, tn, range);
+    if (range >= kRangeEnd) n = node_slow<BATES>(C, tn);
+    return n;
 }
 
 // One strike's node value from the strike-free part: Im(e^Z) / u / t^2 =
@@ -520,13 +700,17 @@ __device__ __forceinline__ NodeCf node_cf(const CfConsts& C, double tn) {
 // LIVE_IN_W: w already carries the liveness (NaN where the node is not live,
 // see node_w_live), as the run cache stores it; the value is then 0 exactly
 // where the explicit test gives 0.
+static __device__ __noinline__ double sin_slow(double ux, double a, double w) {
+    const double nq = rint(ux * 0.15915494309189535);  // 1 / (2 pi)
+    const double uxr = fma(-nq, 2.4492935982947064e-16, fma(-nq, 6.283185307179586, ux));
+    return __dmul_rn(sin(__dadd_rn(a, uxr)), w);
+}
 template <bool LIVE_IN_W = false>
 __device__ __forceinline__ double node_finish_w(double x, double tn, double w, double a, double u) {
     const double ux = __dmul_rn(u, x);
-    const double nq = rint(ux * 0.15915494309189535);  // 1 / (2 pi)
-    const double uxr = fma(-nq, 2.4492935982947064e-16, fma(-nq, 6.283185307179586, ux));
-    const double v = __dmul_rn(sin(__dadd_rn(a, uxr)), w);
-    const bool ok = (LIVE_IN_W || ((tn > 0.0) && (u >= 1e-12))) && isfinite(v);
+    double v = sin_node(ux, a, w);
+    if (max(node_range(ux), node_range(a)) >= kRangeEnd) v = sin_slow(ux, a, w);
+    const bool ok = (LIVE_IN_W || u >= 1e-12) && isfinite(v);
     return ok ? v : 0.0;
 }
 

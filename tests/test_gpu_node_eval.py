@@ -37,3 +37,23 @@ def test_nodes_beyond_correlation_one(ope, oracle, rho, which):
     a, b = got[0, 9:39], ref[0, 9:39]
     assert np.array_equal(np.isfinite(a), np.isfinite(b))
     assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(b))
+
+
+@pytest.mark.gpu
+def test_nodes_beyond_the_fast_functions_range(ope, oracle):
+    """A jump mean of -2^47: the jump factor's phase passes 2^45 on the nodes
+    with u > 1/4, below which the fast functions apply (P2; both evaluate
+    cos and sin of the same rounded phase).  Same bar as above."""
+    con = W.c1().contracts[37:38]
+    par = np.array((0.04, 1.5, 0.04, 0.5, -0.7, 0.8, -2.0 ** 47, 0.1))
+    got, _ = ope.trace_integral(ope.MODEL_BATES, con, par, 1, tol=1e-10)
+    ref, _ = oracle.trace_integral(con, par, True, 1, 1e-10)
+    a, b = got[0, 9:39], ref[0, 9:39]
+    assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(b))
+    # a phase of 2^47 u in the final sine: its last place alone moves it by
+    # more than 1e-2, so only its magnitude is bounded, by the node weights
+    big = con.copy()
+    big["rate"] = 2.0 ** 47 / big["expiry"]
+    ref0, _ = oracle.trace_integral(con, par[:5], False, 1, 1e-10)
+    got, _ = ope.trace_integral(ope.MODEL_HESTON, big, par[:5], 1, tol=1e-10)
+    assert np.all(np.isfinite(got[0])) and np.max(np.abs(got[0, 9:39])) <= 1e3 * np.max(np.abs(ref0[0, 9:39]))
