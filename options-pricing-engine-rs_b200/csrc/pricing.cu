@@ -171,8 +171,8 @@ __device__ __forceinline__ void run_unit(long long c, int which, const ope_contr
         const size_t idx = (size_t)(2 * c + which) * sink.n_slots + slot;
         double* dst = sink.panels + idx * (2 * kMaxPanels);
         for (int i = lane; i <= nb; i += 32) {
-            dst[2 * i] = L.a[i];
-            dst[2 * i + 1] = L.b[i];
+            dst[2 * i] = L.ab[i].x;
+            dst[2 * i + 1] = L.ab[i].y;
         }
         if (lane == 0) sink.nbis[idx] = nb;
         __syncwarp();  // the list is read before the next unit rewrites it

@@ -63,11 +63,10 @@ static __constant__ double c_gk_wg[16] = {
     0.0};
 
 // One warp's live-panel list (structure of arrays, 6400 bytes).
-struct PanelStore {
+struct alignas(16) PanelStore {
     unsigned long long ekey[kMaxPanels];  // error as IEEE bits (total_cmp order for err >= 0)
     double k[kMaxPanels];
-    double a[kMaxPanels];
-    double b[kMaxPanels];
+    double2 ab[kMaxPanels];
 };
 
 // Per-lane quadrature constants, loaded once per warp.
@@ -79,6 +78,9 @@ struct LaneRule {
     // the one whose product the lane keeps (G7 if lane bit 3 is set) and the
     // one whose product it sends to lane ^ 8
     double wkeep, wsend;
+    // word of the panel list's entry 0 this lane moves on a swap_remove
+    // (lanes 0-3: ekey, k, a, b), as a byte offset, and that word's stride
+    unsigned copy_at, copy_by;
 };
 
 __device__ __forceinline__ LaneRule lane_rule(int lane) {
@@ -91,29 +93,25 @@ __device__ __forceinline__ LaneRule lane_rule(int lane) {
     R.half = lane >> 4;
     R.wkeep = (lane & 8) ? R.wg : R.wk;
     R.wsend = (lane & 8) ? R.wk : R.wg;
+    R.copy_at = lane == 0 ? 0u : 1600u * (unsigned)min(lane, 2) + (lane == 3 ? 8u : 0u);
+    R.copy_by = lane < 2 ? 8u : 16u;
     return R;
 }
 
-// K15 and G7 sums of both children, in every lane.  A reduce-scatter over
-// each half-warp: at the first exchange (lanes i and i^8) the lanes with bit
-// 3 clear keep a K15 partial sum and those with it set a G7 partial sum (each
+// K15 and G7 sums of each half-warp's child.  A reduce-scatter over the
+// half-warp: at the first exchange (lanes i and i^8) the lanes with bit 3
+// clear keep a K15 partial sum and those with it set a G7 partial sum (each
 // lane sends the product its partner keeps), and three more xor levels
 // finish each sum with one shuffle per level.  Every lane adds the same two
 // partial sums at each level (commuted in its partner), so all lanes of a
-// quarter hold bit-identical totals, summed in the pairing order (8, 4, 2, 1);
-// lanes 0, 8, 16 and 24 then broadcast the four totals.
-__device__ __forceinline__ void gk_sums(double f, const LaneRule& R, double& Kl, double& Gl, double& Kr,
-                                        double& Gr) {
+// quarter hold bit-identical totals, summed in the pairing order (8, 4, 2, 1):
+// K15 in the lanes with bit 3 clear, G7 in the others.
+__device__ __forceinline__ double gk_sums(double f, const LaneRule& R) {
     const unsigned FULL = 0xffffffffu;
-    double v = R.wkeep * f;
-    v += __shfl_xor_sync(FULL, R.wsend * f, 8);
-    v += __shfl_xor_sync(FULL, v, 4);
-    v += __shfl_xor_sync(FULL, v, 2);
-    v += __shfl_xor_sync(FULL, v, 1);
-    Kl = __shfl_sync(FULL, v, 0);
-    Gl = __shfl_sync(FULL, v, 8);
-    Kr = __shfl_sync(FULL, v, 16);
-    Gr = __shfl_sync(FULL, v, 24);
+    double v = fma(R.wkeep, f, __shfl_xor_sync(FULL, __dmul_rn(R.wsend, f), 8));
+    v = __dadd_rn(v, __shfl_xor_sync(FULL, v, 4));
+    v = __dadd_rn(v, __shfl_xor_sync(FULL, v, 2));
+    return __dadd_rn(v, __shfl_xor_sync(FULL, v, 1));
 }
 
 // The run cache: node_cf's values at the panels that the contracts of one
@@ -184,16 +182,24 @@ __device__ __forceinline__ void run_cache_discard(RunCacheWarp& rc, int lane) {
 // and inlined: no code); the QAG trace kernel (trace.cu) records every step.
 //   first(lane, f, k0, e0): the first panel [0, 1] (f: this lane's integrand
 //     value, lanes 0-14 hold the 15 nodes);
-//   step(j, lane, f, a, b, ew, kl, el, kr, er, err, total): bisection j of
-//     panel [a, b] (error estimate ew) into children with K and error
-//     estimates kl, el, kr, er, and the running error and total after it.
+//   step(j, lane, f, a, b, ew, k, e, kx, ex, err, total): bisection j of a
+//     panel of error estimate ew; [a, b], k and e are this half-warp's child,
+//     its K and error estimate, kx and ex the other half's; then the running
+//     error and total after it (k, kx, total: in the lanes with bit 3 clear).
 struct NoTrace {
     __device__ __forceinline__ void first(int, double, double, double) const {}
     __device__ __forceinline__ void step(int, int, double, double, double, double, double, double, double, double,
                                          double, double) const {}
 };
 
-// Returns the integral (identical in every lane).  `nbis` receives the
+// What bounds a step besides its node: issue slots.  Each half-warp keeps its
+// own child's sums and writes its own list entry (one leader lane each), and
+// the four words of a swap_remove move in one load and one store; with both
+// children's values in every lane and lane 0 writing the whole list, the
+// 262k-contract Bates batch took 10.17 ms instead of 9.79, the run kernel's
+// 1.46M-contract grids 32.4 ms instead of 27.2.
+//
+// Returns the integral (in the lanes with bit 3 clear).  `nbis` receives the
 // number of bisections (loop iterations of heston.rs:200-210); the final
 // live-panel list (nbis + 1 entries) is left in L.  The first panel and every
 // bisection go through ONE call site of the integrand, so the (large) inlined
@@ -210,20 +216,19 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
     const unsigned FULL = 0xffffffffu;
     double total = 0.0, err = 0.0;
     int len = 0;
-    // panel under evaluation in this half-warp; first step: [0, 1] on the left half only
-    double pa = 0.0, pb = 1.0;
-    bool active = (R.half == 0) && R.node;
-    double aw = 0.0, bw = 1.0, m = 0.5, kw = 0.0, ew = 0.0;
-    int w = 0;
+    // panel under evaluation in this half-warp; first step: [0, 1] in both
+    // halves, the right half's result unused
+    double pa = 0.0, pb = 1.0, kw = 0.0, ew = 0.0;
+    char* const list = reinterpret_cast<char*>(&L);
     // cache mode of the step (warp-uniform): hit = read entries el_/er_,
     // put = evaluate and store into them; neither = evaluate uncached.  The
-    // first step's panel [0, 1] is entry 0 (read as the left child).
+    // first step's panel [0, 1] is entry 0.
     bool hit = false, put = false;
     int el_ = kNoEntry, er_ = kNoEntry, sw_ = kNoEntry;  // sw_: entry of the bisected panel
     if (CACHED && rc->on) {
         if (rc->n_alloc > 0) {
             hit = true;
-            el_ = 0;
+            el_ = er_ = 0;
         } else if (rc->cap > 0) {
             put = true;
             el_ = 0;
@@ -233,96 +238,69 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
     while (true) {
         const double c = 0.5 * (pa + pb), h = 0.5 * (pb - pa);
         const double tn = __dadd_rn(c, __dmul_rn(h, R.x));
-        // the node's strike-free part: W, A, u (from the tree on a hit)
-        double nw = 0.0, na = 0.0, nu = 0.0;
+        // the node's strike-free part: W, A, u (from the tree on a hit).  The
+        // pad lanes 15 and 31 evaluate the panel's centre; their weights are 0.
+        double nw, na, nu;
         if (CACHED && hit) {
-            if (active) {
-                const size_t i = (size_t)(R.half ? er_ : el_) * 16 + (lane & 15);
-                nw = __ldcg(rc->w + i);
-                na = __ldcg(rc->a + i);
-                nu = node_u_of(tn);
-            }
+            const size_t i = (size_t)(R.half ? er_ : el_) * 16 + (lane & 15);
+            nw = __ldcg(rc->w + i);
+            na = __ldcg(rc->a + i);
+            nu = node_u_of(tn);
         } else {
-            if (active) {
-                if (CACHED) {
-                    const NodeW nc = node_cf_call<BATES>(C, tn);
-                    nw = nc.w;
-                    na = nc.a;
-                    nu = nc.u;
-                } else {
-                    const NodeCf nc = node_cf<BATES>(C, tn);
-                    nw = node_w(nc);
-                    na = nc.a;
-                    nu = nc.u;
-                }
+            if (CACHED) {
+                const NodeW nc = node_cf_call<BATES>(C, tn);
+                nw = nc.w;
+                na = nc.a;
+                nu = nc.u;
+            } else {
+                const NodeCf nc = node_cf<BATES>(C, tn);
+                nw = node_w(nc);
+                na = nc.a;
+                nu = nc.u;
             }
-            // the half-warps that evaluated a child write its entry, the
-            // pad lane (15 or 31) the 16th element
-            if (CACHED && put && (active || (!R.node && (len > 0 || R.half == 0)))) {
+            // each half-warp writes its child's entry whole, pad lane included
+            if (CACHED && put && (len > 0 || R.half == 0)) {
                 const size_t i = (size_t)(R.half ? er_ : el_) * 16 + (lane & 15);
                 __stcg(rc->w + i, nw);
                 __stcg(rc->a + i, na);
             }
         }
-        const double f = active ? node_finish_w<CACHED>(C.x, tn, nw, na, nu) : 0.0;
-        double Kl, Gl, Kr, Gr;
-        gk_sums(f, R, Kl, Gl, Kr, Gr);
-        if (len == 0) {
-            const double k0 = __dmul_rn(Kl, 0.5), e0 = __dmul_rn(fabs(Kl - Gl), 0.5);
-            if (lane == 0) {
-                L.ekey[0] = (unsigned long long)__double_as_longlong(e0);
-                L.k[0] = k0;
-                L.a[0] = 0.0;
-                L.b[0] = 1.0;
-            }
-            total = k0;
-            err = e0;
-            len = 1;
-            tr.first(lane, f, k0, e0);
-            if (CACHED && rc->on && lane == 0) {
-                rc->slot[0] = (uint16_t)el_;
-                if (put) rc->child[0] = kNoChildren;
-            }
+        const double f = node_finish_w<CACHED>(C.x, tn, nw, na, nu);
+        // K (in the lanes with bit 3 clear) and error of this half's child,
+        // then both children's sums
+        const double v = gk_sums(f, R);
+        const double e = __dmul_rn(fabs(__dsub_rn(v, __shfl_xor_sync(FULL, v, 8))), h), k = __dmul_rn(v, h);
+        const double ex = __shfl_xor_sync(FULL, e, 16), kx = __shfl_xor_sync(FULL, k, 16);
+        const bool first = len == 0;
+        if (first) {
+            total = k;
+            err = e;
+            tr.first(lane, R.half ? 0.0 : f, k, e);
         } else {
-            const double hl = 0.5 * (m - aw), hr = 0.5 * (bw - m);
-            const double kl = __dmul_rn(Kl, hl), el = __dmul_rn(fabs(Kl - Gl), hl);
-            const double kr = __dmul_rn(Kr, hr), er = __dmul_rn(fabs(Kr - Gr), hr);
-            total = __dadd_rn(total, __dsub_rn(__dadd_rn(kl, kr), kw));
-            err = __dadd_rn(err, __dsub_rn(__dadd_rn(el, er), ew));
-            tr.step(len, lane, f, aw, bw, ew, kl, el, kr, er, err, total);
-            if (lane == 0) {
-                const int last = len - 1;
-                if (w != last) {  // swap_remove
-                    L.ekey[w] = L.ekey[last];
-                    L.k[w] = L.k[last];
-                    L.a[w] = L.a[last];
-                    L.b[w] = L.b[last];
-                }
-                L.ekey[last] = (unsigned long long)__double_as_longlong(el);
-                L.k[last] = kl;
-                L.a[last] = aw;
-                L.b[last] = m;
-                L.ekey[len] = (unsigned long long)__double_as_longlong(er);
-                L.k[len] = kr;
-                L.a[len] = m;
-                L.b[len] = bw;
-                if (CACHED && rc->on) {
-                    if (w != last) rc->slot[w] = rc->slot[last];
-                    rc->slot[last] = (uint16_t)el_;
-                    rc->slot[len] = (uint16_t)er_;
-                    if (put) {
-                        rc->child[el_] = kNoChildren;
-                        rc->child[er_] = kNoChildren;
-                        rc->child[sw_] = (uint32_t)el_ | ((uint32_t)er_ << 16);
-                    } else if (hit) {
-                        // the children's own child words, read when they are bisected
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(rc->child + el_));
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(rc->child + er_));
-                    }
+            total = __dadd_rn(total, __dsub_rn(__dadd_rn(k, kx), kw));
+            err = __dadd_rn(err, __dsub_rn(__dadd_rn(e, ex), ew));
+            tr.step(len, lane, f, pa, pb, ew, k, e, kx, ex, err, total);
+        }
+        // push(left) over the list's last slot (its panel was bisected, or
+        // moved to the bisected one's slot below), push(right) behind it
+        if ((lane & 15) == 0 && !(first && R.half)) {
+            const int at = first ? 0 : len - 1 + R.half;
+            L.ekey[at] = (unsigned long long)__double_as_longlong(e);
+            L.k[at] = k;
+            L.ab[at] = make_double2(pa, pb);
+            if (CACHED && rc->on) {
+                const int own = R.half ? er_ : el_;
+                rc->slot[at] = (uint16_t)own;
+                if (put) {
+                    rc->child[own] = kNoChildren;
+                    if (!first && !R.half) rc->child[sw_] = (uint32_t)el_ | ((uint32_t)er_ << 16);
+                } else if (hit && !first) {
+                    // the child's own child word, read when it is bisected
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(rc->child + own));
                 }
             }
-            ++len;
         }
+        ++len;
         __syncwarp();
         if (!(err > tol && len < kMaxPanels)) break;
         if (!ope_check(len < kMaxPanels, CHK_PANEL_COUNT)) break;
@@ -350,19 +328,21 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
             bi = (int)mi - 1;
         }
         if (!ope_check(bi >= 0 && bi < len, CHK_PANEL_INDEX)) bi = 0;
-        w = bi;
+        const int w = bi, last = len - 1;
         ew = __longlong_as_double((long long)best);
         kw = L.k[w];
-        aw = L.a[w];
-        bw = L.b[w];
-        m = 0.5 * (aw + bw);
-        pa = R.half ? m : aw;
-        pb = R.half ? bw : m;
-        active = R.node;
+        const double2 ab = L.ab[w];
+        const double m = 0.5 * (ab.x + ab.y);
+        pa = R.half ? m : ab.x;
+        pb = R.half ? ab.y : m;
+        unsigned long long word = 0;
+        if (lane < 4) word = *reinterpret_cast<const unsigned long long*>(list + (R.copy_at + last * R.copy_by));
+        int moved = 0;
         if (CACHED && rc->on) {
             // the children of panel w: in the tree (hit), or new entries (put)
             // while the tree has room for both and w is in it
             sw_ = rc->slot[w];
+            moved = rc->slot[last];
             hit = put = false;
             el_ = er_ = kNoEntry;
             if (sw_ != kNoEntry && !ope_check(sw_ < rc->n_alloc, CHK_RUN_ENTRY)) sw_ = kNoEntry;
@@ -385,7 +365,10 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
                 }
             }
         }
-        __syncwarp();  // every lane has read entry w before lane 0 rewrites it
+        __syncwarp();  // every lane has read entry w before it is overwritten
+        // swap_remove: the last entry takes the bisected one's slot
+        if (lane < 4) *reinterpret_cast<unsigned long long*>(list + (R.copy_at + w * R.copy_by)) = word;
+        if (CACHED && rc->on && lane == 0) rc->slot[w] = (uint16_t)moved;
     }
     *nbis = len - 1;
     return total;

@@ -51,9 +51,11 @@ struct StepRecorder {
     __device__ __forceinline__ void first(int lane, double f, double k0, double e0) const {
         put(0, lane, f, 0.0, 1.0, 0.0, k0, e0, 0.0, 0.0, e0, k0);
     }
-    __device__ __forceinline__ void step(int j, int lane, double f, double a, double b, double ew, double kl,
-                                         double el, double kr, double er, double err, double total) const {
-        put(j, lane, f, a, b, ew, kl, el, kr, er, err, total);
+    // a, k, e: this half-warp's child, kx, ex: the other half's; b of the
+    // bisected panel is the right child's end
+    __device__ __forceinline__ void step(int j, int lane, double f, double a, double b, double ew, double k, double e,
+                                         double kx, double ex, double err, double total) const {
+        put(j, lane, f, a, __shfl_sync(0xffffffffu, b, 16), ew, k, e, kx, ex, err, total);
     }
 };
 
