@@ -105,6 +105,123 @@ __device__ __forceinline__ double atan2_node(double y, double x) {
     return copysign(r, y);
 }
 
+// arg(x + iy) for the node evaluation's Log A, by a rotation: the difference of
+// the high words of |y| and |x| is log2 |y/x| to within 0.09, which with the
+// two signs picks one of 84 directions K (bins half an octave wide, so K lies
+// within 0.111 of the angle; K = 0 and pi/2 beyond 2^(+-4.75)); turned by -K,
+// t = (y cos K - x sin K)/(x cos K + y sin K), arg = K + atan t, atan t =
+// t + t s P(s), s = t^2, P the degree-5 Chebyshev interpolant (8.8e-19 absolute).  Without
+// it (atan2_node's octant reduction) a node makes seven selects, three
+// comparisons, three additions and five polynomial steps more.  x = y = 0 and
+// non-finite arguments give NaN or a finite angle; in the node evaluation
+// those come only with a 1/|N|^2 that is not finite and drops the node.
+struct alignas(16) ArgDir {
+    double c, s, k, pad;
+};
+static __device__ const ArgDir g_arg_tab[84] = {
+    {1.0, 0.0, 0.0, 0.0},
+    {0.9990248656871402, 0.044151078568834795, 0.04416543524608704, 0.0},
+    {0.9980525784828885, 0.06237828615518053, 0.06241880999595735, 0.0},
+    {0.9961164901835046, 0.08804509063256238, 0.08815924263434795, 0.0},
+    {0.9922778767136676, 0.12403473458920845, 0.12435499454676144, 0.0},
+    {0.9847319278346619, 0.17407765595569785, 0.17496904566568885, 0.0},
+    {0.9701425001453319, 0.24253562503633297, 0.24497866312686414, 0.0},
+    {0.9428090415820634, 0.3333333333333333, 0.3398369094541219, 0.0},
+    {0.8944271909999159, 0.4472135954999579, 0.4636476090008061, 0.0},
+    {0.816496580927726, 0.5773502691896257, 0.6154797086703873, 0.0},
+    {0.7071067811865476, 0.7071067811865476, 0.7853981633974483, 0.0},
+    {0.5773502691896257, 0.816496580927726, 0.9553166181245093, 0.0},
+    {0.4472135954999579, 0.8944271909999159, 1.1071487177940904, 0.0},
+    {0.3333333333333333, 0.9428090415820634, 1.2309594173407747, 0.0},
+    {0.24253562503633297, 0.9701425001453319, 1.3258176636680326, 0.0},
+    {0.17407765595569785, 0.9847319278346619, 1.3958272811292078, 0.0},
+    {0.12403473458920845, 0.9922778767136676, 1.446441332248135, 0.0},
+    {0.08804509063256238, 0.9961164901835046, 1.4826370841605487, 0.0},
+    {0.06237828615518053, 0.9980525784828885, 1.5083775167989393, 0.0},
+    {0.044151078568834795, 0.9990248656871402, 1.5266308915488096, 0.0},
+    {0.0, 1.0, 1.5707963267948966, 0.0},
+    {-1.0, 0.0, 3.141592653589793, 0.0},
+    {-0.9990248656871402, 0.044151078568834795, 3.0974272183437064, 0.0},
+    {-0.9980525784828885, 0.06237828615518053, 3.079173843593836, 0.0},
+    {-0.9961164901835046, 0.08804509063256238, 3.0534334109554453, 0.0},
+    {-0.9922778767136676, 0.12403473458920845, 3.017237659043032, 0.0},
+    {-0.9847319278346619, 0.17407765595569785, 2.966623607924104, 0.0},
+    {-0.9701425001453319, 0.24253562503633297, 2.896613990462929, 0.0},
+    {-0.9428090415820634, 0.3333333333333333, 2.8017557441356713, 0.0},
+    {-0.8944271909999159, 0.4472135954999579, 2.677945044588987, 0.0},
+    {-0.816496580927726, 0.5773502691896257, 2.5261129449194057, 0.0},
+    {-0.7071067811865476, 0.7071067811865476, 2.356194490192345, 0.0},
+    {-0.5773502691896257, 0.816496580927726, 2.186276035465284, 0.0},
+    {-0.4472135954999579, 0.8944271909999159, 2.0344439357957027, 0.0},
+    {-0.3333333333333333, 0.9428090415820634, 1.9106332362490186, 0.0},
+    {-0.24253562503633297, 0.9701425001453319, 1.8157749899217608, 0.0},
+    {-0.17407765595569785, 0.9847319278346619, 1.7457653724605855, 0.0},
+    {-0.12403473458920845, 0.9922778767136676, 1.695151321341658, 0.0},
+    {-0.08804509063256238, 0.9961164901835046, 1.6589555694292446, 0.0},
+    {-0.06237828615518053, 0.9980525784828885, 1.633215136790854, 0.0},
+    {-0.044151078568834795, 0.9990248656871402, 1.6149617620409837, 0.0},
+    {0.0, 1.0, 1.5707963267948966, 0.0},
+    {1.0, -0.0, 0.0, 0.0},
+    {0.9990248656871402, -0.044151078568834795, -0.04416543524608704, 0.0},
+    {0.9980525784828885, -0.06237828615518053, -0.06241880999595735, 0.0},
+    {0.9961164901835046, -0.08804509063256238, -0.08815924263434795, 0.0},
+    {0.9922778767136676, -0.12403473458920845, -0.12435499454676144, 0.0},
+    {0.9847319278346619, -0.17407765595569785, -0.17496904566568885, 0.0},
+    {0.9701425001453319, -0.24253562503633297, -0.24497866312686414, 0.0},
+    {0.9428090415820634, -0.3333333333333333, -0.3398369094541219, 0.0},
+    {0.8944271909999159, -0.4472135954999579, -0.4636476090008061, 0.0},
+    {0.816496580927726, -0.5773502691896257, -0.6154797086703873, 0.0},
+    {0.7071067811865476, -0.7071067811865476, -0.7853981633974483, 0.0},
+    {0.5773502691896257, -0.816496580927726, -0.9553166181245093, 0.0},
+    {0.4472135954999579, -0.8944271909999159, -1.1071487177940904, 0.0},
+    {0.3333333333333333, -0.9428090415820634, -1.2309594173407747, 0.0},
+    {0.24253562503633297, -0.9701425001453319, -1.3258176636680326, 0.0},
+    {0.17407765595569785, -0.9847319278346619, -1.3958272811292078, 0.0},
+    {0.12403473458920845, -0.9922778767136676, -1.446441332248135, 0.0},
+    {0.08804509063256238, -0.9961164901835046, -1.4826370841605487, 0.0},
+    {0.06237828615518053, -0.9980525784828885, -1.5083775167989393, 0.0},
+    {0.044151078568834795, -0.9990248656871402, -1.5266308915488096, 0.0},
+    {0.0, -1.0, -1.5707963267948966, 0.0},
+    {-1.0, -0.0, -3.141592653589793, 0.0},
+    {-0.9990248656871402, -0.044151078568834795, -3.0974272183437064, 0.0},
+    {-0.9980525784828885, -0.06237828615518053, -3.079173843593836, 0.0},
+    {-0.9961164901835046, -0.08804509063256238, -3.0534334109554453, 0.0},
+    {-0.9922778767136676, -0.12403473458920845, -3.017237659043032, 0.0},
+    {-0.9847319278346619, -0.17407765595569785, -2.966623607924104, 0.0},
+    {-0.9701425001453319, -0.24253562503633297, -2.896613990462929, 0.0},
+    {-0.9428090415820634, -0.3333333333333333, -2.8017557441356713, 0.0},
+    {-0.8944271909999159, -0.4472135954999579, -2.677945044588987, 0.0},
+    {-0.816496580927726, -0.5773502691896257, -2.5261129449194057, 0.0},
+    {-0.7071067811865476, -0.7071067811865476, -2.356194490192345, 0.0},
+    {-0.5773502691896257, -0.816496580927726, -2.186276035465284, 0.0},
+    {-0.4472135954999579, -0.8944271909999159, -2.0344439357957027, 0.0},
+    {-0.3333333333333333, -0.9428090415820634, -1.9106332362490186, 0.0},
+    {-0.24253562503633297, -0.9701425001453319, -1.8157749899217608, 0.0},
+    {-0.17407765595569785, -0.9847319278346619, -1.7457653724605855, 0.0},
+    {-0.12403473458920845, -0.9922778767136676, -1.695151321341658, 0.0},
+    {-0.08804509063256238, -0.9961164901835046, -1.6589555694292446, 0.0},
+    {-0.06237828615518053, -0.9980525784828885, -1.633215136790854, 0.0},
+    {-0.044151078568834795, -0.9990248656871402, -1.6149617620409837, 0.0},
+    {0.0, -1.0, -1.5707963267948966, 0.0}};
+__device__ __forceinline__ double arg_node(double y, double x) {
+    const int hy = __double2hiint(y), hx = __double2hiint(x);
+    constexpr int kBin = 1 << 19, kTop = 19 * (1 << 18);  // half an octave, 4.75 octaves
+    int d = (hy & 0x7fffffff) - (hx & 0x7fffffff);
+    d = min(max(d, -kTop - kBin), kTop);
+    const int at = ((d + kTop + kBin) >> 19) + 21 * (int)((unsigned)hx >> 31) + 42 * (int)((unsigned)hy >> 31);
+    const ArgDir* e = g_arg_tab + at;
+    const double2 cs = __ldg(reinterpret_cast<const double2*>(e));
+    const double t = __dmul_rn(fma(y, cs.x, __dmul_rn(-x, cs.y)), rcp_nr(fma(y, cs.y, __dmul_rn(x, cs.x))));
+    const double s = __dmul_rn(t, t);
+    double p = 0.07444393634796143;
+    p = fma(p, s, -0.0908733606338501);
+    p = fma(p, s, 0.1111108660697937);
+    p = fma(p, s, -0.14285714206116987);
+    p = fma(p, s, 0.19999999999895343);
+    p = fma(p, s, -0.33333333333333287);
+    return __dadd_rn(__ldg(&e->k), fma(__dmul_rn(t, s), p, t));
+}
+
 // log|A|^2 of the node evaluation's Log A: log(v), written for this use
 // (2.4 % off the Bates batch against CUDA's log).  Method (the atanh form of
 // the logarithm of Cody and Waite's manual): v = 2^k m with m in
@@ -140,7 +257,8 @@ __device__ __forceinline__ double log_node(double v) {
 // reciprocal: a = 2^k a' with a'/b near 1 (k from the difference of the high
 // words, so a'/b lies within 2^(+-0.59) of 1), then log(a / b) = k ln 2 +
 // 2 atanh(s), s = (a' - b)/(a' + b), |s| <= 0.2, 2 atanh(s) = 2 s + s w R(w)
-// as in log_node (degree 7, from node_math_coeffs.py); both quotients share
+// as in log_node (degree 7, 1.3e-17 relative, from node_math_coeffs.py); both
+// quotients share
 // rcp(a (a' + b)).  A zero, infinite or NaN a gives a
 // non-finite ia (its callers then drop the node).
 __device__ __forceinline__ double log_ratio(double a, double b, double& ia) {
@@ -152,16 +270,16 @@ __device__ __forceinline__ double log_ratio(double a, double b, double& ia) {
     ia = inv * sum;
     const double s = (as - b) * (inv * a);
     const double w = s * s;
-    double r = 0.13636276006553155;
-    r = fma(r, w, 0.13206135972092153);
-    r = fma(r, w, 0.1538905070069374);
-    r = fma(r, w, 0.18181733015886684);
-    r = fma(r, w, 0.22222223107507075);
-    r = fma(r, w, 0.285714285669182);
-    r = fma(r, w, 0.4000000000000874);
-    r = fma(r, w, 0.6666666666666666);
+    double r = 0.13636279106140137;
+    r = fma(r, w, 0.13204848766326904);
+    r = fma(r, w, 0.15389204025268555);
+    r = fma(r, w, 0.18181729316711426);
+    r = fma(r, w, 0.2222222299253829);
+    r = fma(r, w, 0.2857142857209699);
+    r = fma(r, w, 0.3999999999996081);
+    r = fma(r, w, 0.6666666666666672);
     const double kd = (double)k;
-    return fma(kd, 0.6931471805599453, fma(kd, 2.3190468138462996e-17, fma(s * w, r, 2.0 * s)));
+    return fma(kd, 0.6931471824645996, fma(kd, -1.904654299957768e-09, fma(s * w, r, 2.0 * s)));
 }
 
 // Tables of the node evaluation's own exponential and sine/cosine: 2^(j/64),
@@ -221,70 +339,66 @@ static __device__ const double2 g_cis_tab[64] = {
 // integer, left in the low word of the sum.
 constexpr double kRound = 6755399441055744.0;
 
-// The phases exp_node, cis_node and sin_node take must lie below 2^45 in
-// magnitude (node_range: the largest of them, as the high word without its
-// sign; kRangeEnd: 2^45).  Beyond, where a phase's own ulp passes 2^-8, and
-// for non-finite phases, the node takes node_slow.
-constexpr unsigned kRangeEnd = 2u * 0x42C00000u;
+// The arguments exp_node, cis_node and sin_node take must lie below 2^44 in
+// magnitude (node_range: the high word without its sign; kRangeEnd: 2^44).
+// Beyond, where a phase's own ulp passes 2^-9, and for non-finite arguments,
+// the node takes node_slow.
+constexpr unsigned kRangeEnd = 2u * 0x42B00000u;
 __device__ __forceinline__ unsigned node_range(double x) { return 2u * (unsigned)__double2hiint(x); }
 
 // e^x, branch-free (table-driven after Tang, ACM TOMS 15, 1989): x = k ln2/64
-// + r, |r| <= ln2/128, e^x = 2^(k/64) (1 + r + r^2 P(r)), P the degree-3
-// Chebyshev interpolant of node_math_coeffs.py (4e-18 absolute), ln2/64 split
-// into a double and its remainder.  x below -708 is taken as -708 (3e-308)
-// and above 710 as 710 (infinity or NaN); NaN stays NaN.  In place of CUDA's
+// + r, |r| <= 1.03 ln2/128, e^x = 2^(k/64) (1 + r + r^2 P(r)), P of degree 3
+// (9e-18 absolute, node_math_coeffs.py), ln2/64 split into 21 bits and the
+// rest.  k is held within 2^(-1022) and 2^1024, so an x below -708 gives some
+// 1e-308 instead of 0 and one above 709.8 infinity or NaN.  In place of CUDA's
 // exp on the 262k-contract Bates batch: 11.05 -> 10.61 ms (after cis_node and
 // sin_node); a degree-11 polynomial without the table: 10.96 ms.
 __device__ __forceinline__ double exp_node(double x) {
-    int hx = __double2hiint(x);
-    if (x < -708.0) hx = 0xC0862000;  // the high word of -708
-    hx = min(hx, 0x40863000);         // of 710 (a negative x is a negative int)
-    x = __hiloint2double(hx, __double2loint(x));
-    const double t = fma(x, 92.33248261689366, kRound);  // 64/ln2
-    const int k = __double2loint(t);
+    const double t = fma(x, 92.33245849609375, kRound);  // 64/ln2
+    const int k = min(max(__double2loint(t), -1022 * 64), 1024 * 64);
     const double kd = __dsub_rn(t, kRound);
     const double tab = __ldg(g_exp2_tab + (k & 63));
-    double r = fma(kd, -0.010830424696249145, x);
-    r = fma(kd, -3.623510646634843e-19, r);
-    double q = 0.008333339151693497;
-    q = fma(q, r, 0.04166670739519196);
-    q = fma(q, r, 0.16666666666664534);
-    q = fma(q, r, 0.49999999999985073);
+    double r = fma(kd, -0.010830424726009369, x);
+    r = fma(kd, 2.9760223436840126e-11, r);
+    double q = 0.008333340287208557;
+    q = fma(q, r, 0.04166671633720398);
+    q = fma(q, r, 0.1666666666666286);
+    q = fma(q, r, 0.5);
     q = fma(q, __dmul_rn(r, r), r);
     const double sc = __hiloint2double(__double2hiint(tab) + ((k >> 6) << 20), __double2loint(tab));
     return fma(sc, q, sc);
 }
 
-// m e^{ix}, branch-free: x = k pi/32 + r, |r| <= pi/64, pi/32 split into a
-// double and its remainder, sin r and cos r - 1 from the Chebyshev
-// interpolants of node_math_coeffs.py (1.4e-19 and 2.6e-17 absolute), then
-// the angle sum with the table's (cos, sin) of k pi/32.  Error a rounding or
-// two of 1 per component before the product with m.  In place of CUDA's
-// sincos, with sin_node: 11.98 -> 11.05 ms on the same batch; reduced by pi
-// with two longer polynomials and no table: 11.46 ms.
-__device__ __forceinline__ void cis_node(double m, double x, double& re, double& im) {
+// cos x and sin x, branch-free: x = k pi/32 + r, |r| <= pi/64, pi/32 split into
+// 21 bits and the rest, sin r and cos r - 1 from polynomials (3e-19 and 6e-19
+// absolute, node_math_coeffs.py), then the angle sum with the table's
+// (cos, sin) of k pi/32.  Error a rounding or two of 1 per component.  In place
+// of CUDA's sincos, with sin_node: 11.98 -> 11.05 ms on the same batch; reduced
+// by pi with two longer polynomials and no table: 11.46 ms.
+__device__ __forceinline__ void cis_node(double x, double& re, double& im) {
     const double t = fma(x, 10.185916357881302, kRound);  // 32/pi
     const int k = __double2loint(t);
     const double kd = __dsub_rn(t, kRound);
     const double2 cs = __ldg(g_cis_tab + (k & 63));
-    double r = fma(kd, -0.09817477042468103, x);
-    r = fma(kd, -3.827021247335479e-18, r);
+    double r = fma(kd, -0.09817475080490112, x);
+    r = fma(kd, -1.9619779915655082e-08, r);
     const double w = __dmul_rn(r, r);
-    double a = fma(-0.00019840273845896154, w, 0.008333333324333688);
-    a = fma(a, w, -0.16666666666666546);
+    double a = fma(-0.00019840255845338106, w, 0.008333333322977338);
+    a = fma(a, w, -0.16666666666666413);
     const double sr = fma(__dmul_rn(a, w), r, r);  // sin r
-    double b = fma(-0.001388799249796147, w, 0.041666666585670434);
-    b = fma(b, w, -0.4999999999999892);
+    double b = fma(2.4800567189231515e-05, w, -0.00138888880610466);
+    b = fma(b, w, 0.04166666666656595);
+    b = fma(b, w, -0.5);
     const double cm = __dmul_rn(b, w);  // cos r - 1
-    re = __dmul_rn(m, fma(-cs.y, sr, fma(cs.x, cm, cs.x)));
-    im = __dmul_rn(m, fma(cs.x, sr, fma(cs.y, cm, cs.y)));
+    re = fma(-cs.y, sr, fma(cs.x, cm, cs.x));
+    im = fma(cs.x, sr, fma(cs.y, cm, cs.y));
 }
 
 // sin(x + a) w, branch-free, x taken as exact and reduced before a is added:
 // k the integer nearest (x + a)/pi, r = (x - k pi) + a, |r| <= pi/2 (the first
 // subtraction is one FMA, so it rounds at the size of a, not of x), sin r =
-// r + r s Q(s), s = r^2, Q the degree-7 Chebyshev interpolant (1.3e-18
-// absolute), the sign (-1)^k put on w.
+// r + r s Q(s), s = r^2, Q of degree 7 (3.4e-17 relative), the sign (-1)^k put
+// on w.
 __device__ __forceinline__ double sin_node(double x, double a, double w) {
     const double t = fma(__dadd_rn(x, a), 0.3183098861837907, kRound);  // 1/pi
     const int k = __double2loint(t);
@@ -292,13 +406,13 @@ __device__ __forceinline__ double sin_node(double x, double a, double w) {
     double r = fma(kd, -3.141592653589793, x);
     r = __dadd_rn(fma(kd, -1.2246467991473532e-16, r), a);
     const double s = __dmul_rn(r, r);
-    double q = 2.7314447669863995e-15;
-    q = fma(q, s, -7.643970296798572e-13);
-    q = fma(q, s, 1.6058977312464087e-10);
-    q = fma(q, s, -2.5052107616996182e-08);
-    q = fma(q, s, 2.7557319219163234e-06);
-    q = fma(q, s, -0.00019841269841254974);
-    q = fma(q, s, 0.008333333333333316);
+    double q = 2.7314440856698874e-15;
+    q = fma(q, s, -7.643941903057172e-13);
+    q = fma(q, s, 1.6058976370914024e-10);
+    q = fma(q, s, -2.5052107629086277e-08);
+    q = fma(q, s, 2.755731921990685e-06);
+    q = fma(q, s, -0.00019841269841263388);
+    q = fma(q, s, 0.008333333333333344);
     q = fma(q, s, -0.16666666666666666);
     const double sw = __hiloint2double(__double2hiint(w) ^ (k << 31), __double2loint(w));
     return __dmul_rn(fma(__dmul_rn(q, s), r, r), sw);
@@ -437,23 +551,27 @@ __device__ __forceinline__ void csqrt_node(double zr, double zi, double& dre, do
 //   xi   = (xr, -rs u)                       xi = kappa - i rho sigma phi, phi = u + i phi_im
 //   z    = xi^2 + sigma^2 phi(phi+i)         = (zr0 + zr2 u^2, zi1 u): zr0 = xr^2,
 //                                            zr2 = sigma^2 (1 - rho^2), zi1 = sgn sigma^2 - 2 xr rs
-//   C    = kts ((xi - d) T - 2 Log A)        d = sqrt z, ktst = kts T
-//   D    = nv0 phi(phi+i) (1 - e)/N          nv0 = -v0, phi(phi+i) = u^2 + i sgn u
-//   Re Z = Re C + Re D + z0re                z0re = r T + Re(-Log CF(-i)) for P1, 0 for P2
+//   C    = kts ((xi - d) T - 2 Log A)        d = sqrt z
+//   D    = -v0 phi(phi+i) (1 - e)/(2 N)      phi(phi+i) = u^2 + i sgn u = sgn u (sgn u + i)
+//   Re Z = Re C + Re D + r T + Re(-Log CF(-i)) for P1, Re C + Re D for P2
 //   Im Z = Im C + Im D + rtl u + z0im + (x u mod 2 pi)    x = ln(S/K), rtl = r T [- lambda T comp]
-//   Bates: jump = exp(jr0 - hs2 u^2 + i jmu u);  J = (lt Re jump + jre0, lt Im jump)
+//   Bates: jump = exp(jr0 - hs2 u^2 + i jmu u);  J = lt (jump - 1 - i phi comp)
+// (kept: halves of xr, -rs, zr0, zr2, zi1; ktst = 2 kts T, kts2 = 2 kts; nhv0 =
+// -sgn v0/2; z0re: every real term that is constant over the nodes)
 // The C and D of heston.rs:120-124 are formed without g = (xi - d)/(xi + d):
-// with m = xi - d, p = xi + d and N = p - m e (e = exp(-d T)),
-//   A = (g e - 1)/(g - 1) = N / (2 d)   and, since m p = xi^2 - z = -sigma^2 phi(phi+i),
-//   m (1 - e)/(1 - g e) = m p (1 - e)/N = -sigma^2 phi(phi+i) (1 - e)/N,
-// so sigma^2 cancels in D, |A|^2 = |N|^2/(4 |z|) needs no quotient of its
-// own, and a node takes one complex reciprocal (of N) where the literal
-// sequence takes four.
+// with m = (xi - d)/2, e = exp(-d T), o = 1 - e and N = d + m o (half of
+// (xi + d) - (xi - d) e),
+//   A = (g e - 1)/(g - 1) = N/d   and, since xi^2 - d^2 = -sigma^2 phi(phi+i),
+//   (xi - d) o/(1 - g e) = (xi^2 - d^2) o/(2 N) = -sigma^2 phi(phi+i) o/(2 N),
+// so sigma^2 cancels in D, |A|^2 = |N|^2/|z| needs no quotient of its own, and
+// a node takes one complex reciprocal (of N) where the literal sequence takes
+// four.
 struct CfConsts {
-    double xr, rs, zr0, zr2, zi1, kts, ktst, kts2, nv0, sgn, t, rtl, z0re, z0im;
-    double jr0, hs2, jmu, lt, jre0;
+    double hxr, nhrs, hzr0, hzr2, hzi1, t, kts, ktst, kts2, nhv0, rtl, z0re, z0im;
+    double jr0, hs2, jmu, lt;
+    int sgn_bit;
     // raw values kept for the adjoint chain
-    double kappa, phi_im, sig2, v0s, rt, x, lnm_re, lnm_im, mu_j, comp;
+    double kappa, rs, sgn, phi_im, sig2, v0s, rt, x, lnm_re, lnm_im, mu_j, comp;
 };
 
 // stable_cf at a general complex phi, following heston.rs:113-127's operation
@@ -504,13 +622,16 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
     C.x = log_cr(s / k);  // heston.rs:86, rounded as the platform libm rounds it
     C.phi_im = (which == 0) ? -1.0 : 0.0;
     C.sgn = (which == 0) ? -1.0 : 1.0;
-    C.xr = kappa + C.rs * C.phi_im;
-    C.zr0 = C.xr * C.xr;
-    C.zr2 = C.sig2 * ((1.0 - rho) * (1.0 + rho));
-    C.zi1 = fma(-2.0 * C.xr, C.rs, C.sig2 * C.sgn);
-    C.ktst = C.kts * t;
+    const double xr = kappa + C.rs * C.phi_im;
+    C.hxr = 0.5 * xr;
+    C.nhrs = -0.5 * C.rs;
+    C.hzr0 = 0.5 * (xr * xr);
+    C.hzr2 = 0.5 * (C.sig2 * ((1.0 - rho) * (1.0 + rho)));
+    C.hzi1 = 0.5 * fma(-2.0 * xr, C.rs, C.sig2 * C.sgn);
     C.kts2 = 2.0 * C.kts;
-    C.nv0 = -v0;
+    C.ktst = C.kts2 * t;
+    C.nhv0 = -0.5 * v0 * C.sgn;
+    C.sgn_bit = which == 0 ? (int)0x80000000 : 0;
     double lt = 0.0, mu_j = 0.0, hs2 = 0.0, comp = 0.0;
     if (bates) {
         lt = p[5] * t;
@@ -524,7 +645,6 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
     C.comp = comp;
     C.jr0 = -C.phi_im * mu_j + hs2 * (C.phi_im * C.phi_im);
     C.jmu = mu_j - 2.0 * hs2 * C.phi_im;
-    C.jre0 = lt * (C.phi_im * comp - 1.0);
     C.rtl = C.rt - lt * comp;
     C.lnm_re = 0.0;
     C.lnm_im = 0.0;
@@ -538,8 +658,8 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
         // non-finite parameter -- it is evaluated with the reference's own
         // sequence.  (The regular case skips two complex exponentials, three
         // complex divisions and two complex logarithms per P1 integral.)
-        bool regular = C.xr > 1e-100 && C.xr < 1e100 && C.sig2 > 1e-100 && C.kts < 1e4 &&
-                       C.v0s * C.xr < 1e4 && fabs(C.rt) < 700.0 && t < 1e3;
+        bool regular = xr > 1e-100 && xr < 1e100 && C.sig2 > 1e-100 && C.kts < 1e4 &&
+                       C.v0s * xr < 1e4 && fabs(C.rt) < 700.0 && t < 1e3;
         if (bates) regular = regular && fabs(p[6] + 0.5 * p[7] * p[7]) < 50.0 && fabs(lt) * (comp + 1.0) < 1e4;
         if (regular) {
             C.lnm_re = -C.rt;
@@ -552,7 +672,7 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
             C.lnm_im = -lm.im;
         }
     }
-    C.z0re = -C.rt * C.phi_im + C.lnm_re;
+    C.z0re = (-C.rt * C.phi_im + C.lnm_re) + fma(C.kts, 0.6931471805599453, lt * (C.phi_im * comp - 1.0));
     C.z0im = C.lnm_im;
     return C;
 }
@@ -592,81 +712,87 @@ __device__ __forceinline__ double node_u_of(double tn) {
 }
 
 // FAST: branch-free, with the functions above; `range` receives what decides
-// whether they applied (compare with kRangeEnd): the phases of e^{-dT} and of
-// the jump factor, and the sign of Re z (negative only for |rho| > 1).  Not
-// FAST: CUDA's functions and the square root's other branch.
+// whether they applied (compare with kRangeEnd): the largest of their
+// arguments, and the sign of Re z (negative only for |rho| > 1).  Not FAST:
+// CUDA's functions and the square root's other branch.
 //
-// What bounds it: issue slots.  The form without g (CfConsts above), the
-// merged reciprocals and the third-order refinements took the 1M-contract
-// Bates batch from 51.2 to 47.5 ms (262k contracts: 12.99 to 12.03 ms; the
-// same contracts under Heston 11.45 to 10.52 ms); the own exponential, sine
-// and cosine, with their range tests gathered into one branch per node, took
-// the 262k batches on to 10.17 and 8.95 ms (865 to 662 instructions per warp
-// step, 317 to 252 of them FP64).
+// What bounds it: register-file reads and issue slots (an FMA of three
+// different registers takes 3 cycles of a scheduler's operand reads, of two
+// registers and an immediate 2, an addition or a product 2).  So constants are
+// immediates wherever 21 bits do (node_math_coeffs.py), products are folded
+// into FMAs and per-integral constants, and selects are avoided.  On 262k
+// contracts, Bates / Heston, ms:
+//   12.99 / 11.45  with g = (xi - d)/(xi + d) and CUDA's functions
+//   12.03 / 10.52  C and D without g, merged reciprocals
+//   10.17 /  8.95  own exponential, sine and cosine, one range branch per node
+//    9.79 /  8.64  (the bisection step's bookkeeping, quadrature.cuh)
+//    9.66 /  8.45  21-bit leading coefficients and reductions
+//    9.36 /  7.88  N and o as below, arg_node's rotation, integer clamps in
+//                  exp_node (Heston at 72 registers; 8.12 at 64)
+// Two integrals per warp side by side (128 registers) issue 13 % fewer
+// instructions and read as many registers: 9.61 / 8.60 ms against 9.74 / 8.60.
 template <bool BATES, bool FAST>
 __device__ __forceinline__ NodeCf node_eval(const CfConsts& C, double tn, unsigned& range) {
     double u, itt;  // (1 - t) / t and 1 / ((1 - t) t)
     node_geom(tn, u, itt);
     const double u2 = __dmul_rn(u, u);
-    // xi = (xr, xi_) ; z = xi^2 + sigma^2 phi(phi+i) = (xr^2 + zr2 u^2, zi1 u)
-    const double xi_ = __dmul_rn(-C.rs, u);
-    const double zr = fma(C.zr2, u2, C.zr0), zi = __dmul_rn(C.zi1, u);
-    // d = sqrt z: Re d = sqrt((|z| + Re z) / 2), Im d = Im z / (2 Re d)
+    // xi/2 = (hxr, hxi); z/2, z = xi^2 + sigma^2 phi(phi+i) = (xr^2 + zr2 u^2, zi1 u)
+    const double hxi = __dmul_rn(C.nhrs, u);
+    const double zr = fma(C.hzr2, u2, C.hzr0), zi = __dmul_rn(C.hzi1, u);
+    // d = sqrt z: Re d = sqrt(|z/2| + Re z/2), Im d = (Im z/2) / Re d
     const double zz = fma(zr, zr, __dmul_rn(zi, zi));
-    const double hr = __dmul_rn(__dmul_rn(0.5, zz), rsqrt_nr(zz));  // |z| / 2
-    const double s2 = fma(0.5, FAST ? zr : fabs(zr), hr);
+    const double az = __dmul_rn(zz, rsqrt_nr(zz));  // |z| / 2
+    const double s2 = __dadd_rn(FAST ? zr : fabs(zr), az);
     const double iw = rsqrt_nr(s2);
-    double dre = __dmul_rn(s2, iw), dim = __dmul_rn(__dmul_rn(0.5, zi), iw);
+    double dre = __dmul_rn(s2, iw), dim = __dmul_rn(zi, iw);
     if (!FAST && zr < 0.0) {
         const double w = dre;
         dre = fabs(dim);
         dim = copysign(w, zi);
     }
-    const double mr = __dsub_rn(C.xr, dre), mi = __dsub_rn(xi_, dim);  // m = xi - d
-    const double pr = __dadd_rn(C.xr, dre), pi = __dadd_rn(xi_, dim);  // p = xi + d
-    // e = exp(-d T)
+    const double mr = fma(dre, -0.5, C.hxr), mi = fma(dim, -0.5, hxi);  // m = (xi - d) / 2
+    // e = exp(-d T), o = 1 - e
     const double th = __dmul_rn(-dim, C.t), et = __dmul_rn(-dre, C.t);
-    double er, ei;
+    double em, ec, es;
     if (FAST) {
-        range = max(node_range(th), (unsigned)__double2hiint(zr));  // Re z < 0: above kRangeEnd
-        cis_node(exp_node(et), th, er, ei);
+        cis_node(th, ec, es);
+        em = exp_node(et);
     } else {
-        sincos(th, &ei, &er);
-        const double em = exp(et);
-        er = __dmul_rn(em, er);
-        ei = __dmul_rn(em, ei);
+        sincos(th, &es, &ec);
+        em = exp(et);
     }
-    // N = p - m e
-    const double nr = fma(mi, ei, fma(-mr, er, pr));
-    const double ni = fma(-mr, ei, fma(-mi, er, pi));
+    const double omr = fma(-em, ec, 1.0), omi = __dmul_rn(-em, es);
+    // N = d + m o
+    const double nr = fma(-mi, omi, fma(mr, omr, dre));
+    const double ni = fma(mr, omi, fma(mi, omr, dim));
     const double nn = fma(nr, nr, __dmul_rn(ni, ni));
-    // Log A, A = N / (2 d): |A|^2 = nn / (4 |z|), arg A = arg(N conj(d))
+    // Log A, A = N / d: |A|^2 = nn / (2 az) (the 2 is in z0re), arg A = arg(N conj(d))
     double ia;
-    const double la = log_ratio(nn, __dmul_rn(8.0, hr), ia);
-    const double li = atan2_node(fma(ni, dre, __dmul_rn(-nr, dim)), fma(nr, dre, __dmul_rn(ni, dim)));
-    // D = -v0 phi(phi+i) (1 - e) / N, phi(phi+i) = u (u + i sgn)
-    const double omr = __dsub_rn(1.0, er);
-    const double qr = fma(omr, nr, __dmul_rn(-ei, ni)), qi = fma(-ei, nr, __dmul_rn(-omr, ni));
-    const double s = __dmul_rn(__dmul_rn(C.nv0, u), ia);
-    const double Dr = fma(u, qr, __dmul_rn(-C.sgn, qi)), Di = fma(u, qi, __dmul_rn(C.sgn, qr));
+    const double la = log_ratio(nn, az, ia);
+    const double li = arg_node(fma(ni, dre, __dmul_rn(-nr, dim)), fma(nr, dre, __dmul_rn(ni, dim)));
+    // D = -(v0/2) phi(phi+i) o / N, phi(phi+i) = u (u + i sgn) = sgn u (sgn u + i)
+    const double qr = fma(omr, nr, __dmul_rn(omi, ni)), qi = fma(omi, nr, __dmul_rn(-omr, ni));
+    const double su = __hiloint2double(__double2hiint(u) | C.sgn_bit, __double2loint(u));
+    const double s = __dmul_rn(__dmul_rn(C.nhv0, u), ia);
     // Re, Im Z = kts ((xi - d) T - 2 Log A) + D + z0 + i (r T u)
-    double zre = fma(C.ktst, mr, fma(-C.kts, la, fma(s, Dr, C.z0re)));
-    double zim = fma(C.ktst, mi, fma(-C.kts2, li, fma(s, Di, fma(C.rtl, u, C.z0im))));
+    double zre = fma(C.ktst, mr, fma(-C.kts, la, fma(s, fma(su, qr, -qi), C.z0re)));
+    double zim = fma(C.ktst, mi, fma(-C.kts2, li, fma(s, fma(su, qi, qr), fma(C.rtl, u, C.z0im))));
+    if (FAST) range = max(node_range(et), (unsigned)__double2hiint(zr));  // Re z < 0: above kRangeEnd
     if (BATES) {
         const double tj = __dmul_rn(C.jmu, u), ej = fma(-C.hs2, u2, C.jr0);
-        double jr, ji;
+        double jc, js, je;
         if (FAST) {
-            range = max(range, node_range(tj));
-            cis_node(__dmul_rn(C.lt, exp_node(ej)), tj, jr, ji);
+            range = max(range, max(node_range(tj), node_range(ej)));
+            cis_node(tj, jc, js);
+            je = __dmul_rn(C.lt, exp_node(ej));
         } else {
-            sincos(tj, &ji, &jr);
-            const double je = __dmul_rn(C.lt, exp(ej));
-            jr = __dmul_rn(je, jr);
-            ji = __dmul_rn(je, ji);
+            sincos(tj, &js, &jc);
+            je = __dmul_rn(C.lt, exp(ej));
         }
-        zre = __dadd_rn(zre, __dadd_rn(jr, C.jre0));
-        zim = __dadd_rn(zim, ji);
+        zre = fma(je, jc, zre);
+        zim = fma(je, js, zim);
     }
+    if (FAST) range = max(range, node_range(zre));
     return NodeCf{FAST ? exp_node(zre) : exp(zre), zim, u, itt};
 }
 

@@ -24,17 +24,16 @@
 // Register budget of the pricing kernel: per model, the minimum resident
 // blocks per SM of the 4-warp shape handed to __launch_bounds__ (registers
 // per thread capped at 65536 / (32 * 4 * MINB)); the 1- and 2-warp shapes get
-// 4 / warps times as many blocks, the same 64 registers.  8 for both models:
-// the fastest of 5-9 blocks on each model's full batch (within 2 % of one
-// another; kept per model because the optimum has moved apart and back with
-// changes to the node evaluation).
+// 4 / warps times as many blocks.  262k wing contracts, 8 / 7 blocks (64 / 72
+// registers): Bates 9.36 / 9.40 ms, Heston 8.12 / 7.88 ms.
 #ifndef OPE_KERNEL_MINB_BATES
 #define OPE_KERNEL_MINB_BATES 8
 #endif
 #ifndef OPE_KERNEL_MINB_HESTON
-#define OPE_KERNEL_MINB_HESTON 8
+#define OPE_KERNEL_MINB_HESTON 7
 #endif
-// The same for the run kernel (both models).
+// The same for the run kernel (both models): 8 / 7 blocks 27.1 / 32.8 ms on
+// 1.46M grid contracts.
 #ifndef OPE_RUNS_MINB
 #define OPE_RUNS_MINB 8
 #endif
