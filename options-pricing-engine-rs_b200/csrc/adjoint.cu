@@ -13,14 +13,13 @@
 //      warps pull chunks from that list; the 15 nodes of each panel are
 //      spread over the 32 lanes, each lane recomputes the CF at its node and
 //      runs the backward pass (cf_adjoint.cuh), accumulating all parameter
-//      derivatives at once; for P1 one extra work item of the first chunk
-//      evaluates the normaliser's dLog CF(-i)/dp; a warp reduction finishes
-//      each chunk's partial sums.  Chunking spreads a long integral over
+//      derivatives at once; a warp reduction finishes each chunk's partial
+//      sums.  Chunking spreads a long integral over
 //      several warps, which matters when few integrals are left (the tail of
 //      a calibration): the LM batch ran 126.5 -> 94.4 ms at unchanged
 //      gradient throughput;
-//   3. a per-contract combine: the chunks' partial sums in chunk order, the
-//      P1 normaliser term, then ad.rs:713-730, d price = S e^{-qT} dI1/pi -
+//   3. a per-contract combine: the chunks' partial sums in chunk order, then
+//      ad.rs:713-730, d price = S e^{-qT} dI1/pi -
 //      K e^{-rT} dI2/pi for calls and puts alike (parity terms do not depend
 //      on the model parameters).
 // Splitting the primal from the backward pass keeps each kernel's code small
@@ -35,13 +34,20 @@
 #include "quadrature.cuh"
 
 // Minimum resident blocks per SM for the backward kernels' __launch_bounds__
-// (caps registers per thread at 65536 / (128 * OPE_GRAD_MINB)): 5, i.e. 96
-// registers.  The kernel time is flat from 4 to 7 blocks (within 0.5 % on the
-// 262k-contract Bates gradient, 1 % on the Heston one), but at 7 blocks (72
-// registers) its spills overflow L1: 274 MB of DRAM writes per 65,536 Bates
-// contracts against 12 MB at 5 blocks (ncu, one launch).
-#ifndef OPE_GRAD_MINB
-#define OPE_GRAD_MINB 5
+// (caps registers per thread at 65536 / (128 * blocks)): the fastest of 3-6 on
+// 32,768 Bates contracts, price + gradient 2.338 / 2.266 / 2.297 / 2.301 ms,
+// and on the 19,200-quote Heston Jacobian, 0.761 / 0.755 / 0.734 / 0.738 ms.
+//
+// What bounds the backward pass is what bounds the pricing node (cf_device.cuh):
+// operand reads and issue slots.  The form without g, the own functions, one
+// linear combination per chunk instead of per node, and no normaliser term
+// took k_grad_backward<Bates> from 1.26 to 0.83 ms on those 32,768 contracts,
+// and k_greeks_backward<Heston> from 95 to 74 us on 7,680.
+#ifndef OPE_GRAD_MINB_BATES
+#define OPE_GRAD_MINB_BATES 4
+#endif
+#ifndef OPE_GRAD_MINB_HESTON
+#define OPE_GRAD_MINB_HESTON 5
 #endif
 
 namespace ope {
@@ -76,8 +82,7 @@ struct BackScratch {
     uint32_t* unit_base;        // first chunk slot of each integral
     uint8_t* nch;               // chunks of each integral (0 on masked surfaces)
     unsigned long long* work;   // chunk list: integral * 8 + chunk, in slot order
-    double* part;               // per chunk slot: dim derivative sums, then sum W (re, im)
-    double* normd;              // per contract: the P1 normaliser's dLog CF(-i)/dp (re, im)
+    double* part;               // per chunk slot: the derivative sums
     unsigned long long* count;  // [0] chunk slots allocated, [1] queue head
 };
 
@@ -123,13 +128,13 @@ __global__ void k_grad_chunks(long long n, const int64_t* __restrict__ surf_off,
 }
 
 template <bool BATES>
-__global__ void __launch_bounds__(128, OPE_GRAD_MINB) k_grad_backward(const ope_contract* __restrict__ con, long long n,
+__global__ void __launch_bounds__(128, BATES ? OPE_GRAD_MINB_BATES : OPE_GRAD_MINB_HESTON) k_grad_backward(const ope_contract* __restrict__ con, long long n,
                                                       const int64_t* __restrict__ surf_off, long long n_surf,
                                                       const int32_t* __restrict__ param_idx,
                                                       const double* __restrict__ params, PanelSink src,
                                                       BackScratch B) {
     constexpr int DIM = BATES ? 8 : 5;
-    __shared__ double s_norm[4][16];  // per warp: the P1 normaliser's dLog CF(-i)/dp (complex, DIM <= 8)
+    __shared__ CfConsts s_consts[4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const LaneRule R = lane_rule(lane);
     const unsigned long long n_work = *(volatile unsigned long long*)B.count;  // final: set by k_grad_chunks
@@ -150,8 +155,12 @@ __global__ void __launch_bounds__(128, OPE_GRAD_MINB) k_grad_backward(const ope_
 #pragma unroll
         for (int i = 0; i < DIM; ++i) pl[i] = __ldg(p + i);
         const ope_contract* cp = con + c;
-        const CfConsts C = make_consts(__ldg(&cp->spot), __ldg(&cp->strike), __ldg(&cp->expiry), __ldg(&cp->rate),
-                                       pl, BATES, which);
+        const CfConsts Cl = make_consts(__ldg(&cp->spot), __ldg(&cp->strike), __ldg(&cp->expiry), __ldg(&cp->rate),
+                                        pl, BATES, which);
+        __syncwarp();
+        if (lane == 0) s_consts[warp] = Cl;
+        __syncwarp();
+        const CfConsts& C = s_consts[warp];
         const GradParams G = make_grad_params(pl, BATES);
         int slot = src.slot ? __ldg(src.slot + s) : 0;
         if (!ope_check(slot >= 0 && slot < src.n_slots, CHK_SLOT)) slot = 0;
@@ -161,67 +170,48 @@ __global__ void __launch_bounds__(128, OPE_GRAD_MINB) k_grad_backward(const ope_
         const int p0 = chunk * kChunkPanels, p1 = min(len, p0 + kChunkPanels);
         const double* P = src.panels + pidx * (2 * kMaxPanels) + 2 * p0;
         double acc[DIM];
+        const int items = 15 * max(p1 - p0, 0);
+        for (bool fast = true;; fast = false) {
+            double sum[DIM];
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) acc[k] = 0.0;
-        double sw_re = 0.0, sw_im = 0.0;
-        const bool with_norm = which == 0 && chunk == 0;
-        const int total = 15 * max(p1 - p0, 0);
-        const int items = total + (with_norm ? 1 : 0);
-        for (int base = 0; base < items; base += 32) {
-            const int idx = base + lane;
-            const int pi = idx / 15, j = idx - 15 * (idx / 15);
-            const double xj = __shfl_sync(0xffffffffu, R.x, j & 15);
-            const double wj = __shfl_sync(0xffffffffu, R.wk, j & 15);
-            if (idx < items) {
-                const bool normaliser = idx == total;
-                double tn = 0.0, hw = 0.0, u = 0.0, itt = 0.0;
-                if (!normaliser) {
-                    const double a = __ldg(P + 2 * pi), b = __ldg(P + 2 * pi + 1);
-                    const double cc = 0.5 * (a + b), h = 0.5 * (b - a);
-                    tn = __dadd_rn(cc, __dmul_rn(h, xj));
-                    hw = h * wj;
-                    const double omt = 1.0 - tn;
-                    itt = rcp_nr(omt * tn);  // 1 / ((1 - t) t), as the pricing node evaluation
-                    u = (omt * omt) * itt;   // (1 - t) / t
-                }
-                C2 dz[8];
-                const C2 Z = exponent_and_grad<BATES>(C, G, u, dz);
-                if (normaliser) {
+            for (int k = 0; k < DIM; ++k) sum[k] = 0.0;
+            for (int base = 0; base < items; base += 32) {
+                const int idx = base + lane;
+                const int pi = idx / 15, j = idx - 15 * (idx / 15);
+                const double xj = __shfl_sync(0xffffffffu, R.x, j & 15);
+                const double wj = __shfl_sync(0xffffffffu, R.wk, j & 15);
+                if (idx < items) {
+                    const double2 ab = __ldg(reinterpret_cast<const double2*>(P) + pi);
+                    const double cc = 0.5 * (ab.x + ab.y), h = 0.5 * (ab.y - ab.x);
+                    const double tn = __dadd_rn(cc, __dmul_rn(h, xj));
+                    if (!(fast && node_sums<BATES, true>(C, G, tn, h * wj, sum))) {
+                        double g[DIM];
+                        node_sums_slow<BATES>(C, G, tn, h * wj, g);
 #pragma unroll
-                    for (int k = 0; k < DIM; ++k) { s_norm[warp][2 * k] = dz[k].re; s_norm[warp][2 * k + 1] = dz[k].im; }
-                } else {
-                    node_accumulate<BATES>(Z, dz, (tn > 0.0) && (u >= 1e-12), itt, hw, acc, sw_re, sw_im);
+                        for (int k = 0; k < DIM; ++k) sum[k] += g[k];
+                    }
                 }
             }
-        }
+            bool finite = true;
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) acc[k] = warp_sum(acc[k]);
-        sw_re = warp_sum(sw_re);
-        sw_im = warp_sum(sw_im);
-        __syncwarp();
+            for (int k = 0; k < DIM; ++k) {
+                acc[k] = warp_sum(sum[k]);
+                finite = finite && isfinite(acc[k]);
+            }
+            if (finite || !fast) break;  // else each node again, dropping the terms that are not finite
+        }
         if (lane == 0) {
-            double* out = B.part + w * (DIM + 2);
+            heston_chain(G, acc);
+            double* out = B.part + w * DIM;
 #pragma unroll
             for (int k = 0; k < DIM; ++k) out[k] = acc[k];
-            out[DIM] = sw_re;
-            out[DIM + 1] = sw_im;
-            if (with_norm) {
-#pragma unroll
-                for (int k = 0; k < 2 * DIM; ++k) B.normd[c * 2 * DIM + k] = s_norm[warp][k];
-            }
         }
-        __syncwarp();  // s_norm is read before the next work item rewrites it
     }
 }
 
 // ad.rs:713-730 per contract; contracts of masked surfaces are left untouched.
 // Each integral's derivative is the sum of its chunks' partial sums, in chunk
-// order.  For P1 the normaliser term -dLog CF(-i)/dp * sum W (constant over
-// the integral; zero up to rounding for a regular normaliser, ad.rs:705-706
-// carries it through the Dual division) is applied here; where it is not
-// finite (e.g. kappa < rho sigma puts xi + d = 0 at phi = -i), every P1 node's
-// derivative is non-finite in the reference, so every node is dropped
-// (ad.rs:679-682) and the component is 0.
+// order.
 template <int DIM>
 __global__ void k_grad_combine(const ope_contract* __restrict__ con, long long n, const int64_t* __restrict__ surf_off,
                                long long n_surf, const int32_t* __restrict__ param_idx,
@@ -237,24 +227,13 @@ __global__ void k_grad_combine(const ope_contract* __restrict__ con, long long n
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
         const long long u = 2 * c + which;
-        const double* part = B.part + (size_t)B.unit_base[u] * (DIM + 2);
+        const double* part = B.part + (size_t)B.unit_base[u] * DIM;
         const int nc = B.nch[u];
-        double sw_re = 0.0, sw_im = 0.0;
 #pragma unroll
         for (int k = 0; k < DIM; ++k) d[which][k] = 0.0;
-        for (int j = 0; j < nc; ++j) {
+        for (int j = 0; j < nc; ++j)
 #pragma unroll
-            for (int k = 0; k < DIM; ++k) d[which][k] += part[j * (DIM + 2) + k];
-            sw_re += part[j * (DIM + 2) + DIM];
-            sw_im += part[j * (DIM + 2) + DIM + 1];
-        }
-        if (which == 0) {
-#pragma unroll
-            for (int k = 0; k < DIM; ++k) {
-                const C2 dl = c2(B.normd[c * 2 * DIM + 2 * k], B.normd[c * 2 * DIM + 2 * k + 1]);
-                d[0][k] = (isfinite(dl.re) && isfinite(dl.im)) ? d[0][k] - (dl * c2(sw_re, sw_im)).im : 0.0;
-            }
-        }
+            for (int k = 0; k < DIM; ++k) d[which][k] += part[j * DIM + k];
     }
     const ope_contract& cp = con[c];
     const double PI = 3.14159265358979323846;
@@ -269,13 +248,14 @@ __global__ void k_grad_combine(const ope_contract* __restrict__ con, long long n
 // node value), a warp sum per chunk.  One parameter set per contract, as the
 // reference's AD Greeks take (ad.rs:736-865).
 template <bool BATES>
-__global__ void __launch_bounds__(128, OPE_GRAD_MINB) k_greeks_backward(const ope_contract* __restrict__ con, long long n,
+__global__ void __launch_bounds__(128, BATES ? OPE_GRAD_MINB_BATES : OPE_GRAD_MINB_HESTON) k_greeks_backward(const ope_contract* __restrict__ con, long long n,
                                                         const int64_t* __restrict__ surf_off, long long n_surf,
                                                         const int32_t* __restrict__ param_idx,
                                                         const double* __restrict__ params, PanelSink src,
                                                         BackScratch B) {
     constexpr int DIM = BATES ? 8 : 5;
-    const int lane = threadIdx.x & 31;
+    __shared__ CfConsts s_consts[4];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const LaneRule R = lane_rule(lane);
     const unsigned long long n_work = *(volatile unsigned long long*)B.count;  // final: set by k_grad_chunks
     while (true) {
@@ -296,8 +276,11 @@ __global__ void __launch_bounds__(128, OPE_GRAD_MINB) k_greeks_backward(const op
         for (int i = 0; i < DIM; ++i) pl[i] = __ldg(p + i);
         const ope_contract* cp = con + c;
         const double r = __ldg(&cp->rate);
-        const CfConsts C = make_consts(__ldg(&cp->spot), __ldg(&cp->strike), __ldg(&cp->expiry), r, pl, BATES, which);
-        const double is2 = 1.0 / (pl[3] * pl[3]);
+        const CfConsts Cl = make_consts(__ldg(&cp->spot), __ldg(&cp->strike), __ldg(&cp->expiry), r, pl, BATES, which);
+        __syncwarp();
+        if (lane == 0) s_consts[warp] = Cl;
+        __syncwarp();
+        const CfConsts& C = s_consts[warp];
         const double lambda = BATES ? pl[5] : 0.0;
         int slot = src.slot ? __ldg(src.slot + s) : 0;
         if (!ope_check(slot >= 0 && slot < src.n_slots, CHK_SLOT)) slot = 0;
@@ -307,28 +290,36 @@ __global__ void __launch_bounds__(128, OPE_GRAD_MINB) k_greeks_backward(const op
         const int p0 = chunk * kChunkPanels, p1 = min(len, p0 + kChunkPanels);
         const double* P = src.panels + pidx * (2 * kMaxPanels) + 2 * p0;
         double acc[7];
-#pragma unroll
-        for (int k = 0; k < 7; ++k) acc[k] = 0.0;
         const int items = 15 * max(p1 - p0, 0);
-        for (int base = 0; base < items; base += 32) {
-            const int idx = base + lane;
-            const int pi = idx / 15, j = idx - 15 * (idx / 15);
-            const double xj = __shfl_sync(0xffffffffu, R.x, j & 15);
-            const double wj = __shfl_sync(0xffffffffu, R.wk, j & 15);
-            if (idx < items) {
-                const double a = __ldg(P + 2 * pi), b = __ldg(P + 2 * pi + 1);
-                const double cc = 0.5 * (a + b), h = 0.5 * (b - a);
-                const double tn = __dadd_rn(cc, __dmul_rn(h, xj));
-                const double omt = 1.0 - tn;
-                const double itt = rcp_nr(omt * tn);  // 1 / ((1 - t) t)
-                const double u = node_u(omt, tn, itt);
-                C2 Zv, ZT;
-                const C2 Z = exponent_and_greeks<BATES>(C, u, r, lambda, is2, Zv, ZT);
-                greeks_accumulate(Z, Zv, ZT, u, C.t, (tn > 0.0) && (u >= 1e-12), itt, h * wj, acc);
-            }
-        }
+        for (bool fast = true;; fast = false) {
+            double sum[7];
 #pragma unroll
-        for (int k = 0; k < 7; ++k) acc[k] = warp_sum(acc[k]);
+            for (int k = 0; k < 7; ++k) sum[k] = 0.0;
+            for (int base = 0; base < items; base += 32) {
+                const int idx = base + lane;
+                const int pi = idx / 15, j = idx - 15 * (idx / 15);
+                const double xj = __shfl_sync(0xffffffffu, R.x, j & 15);
+                const double wj = __shfl_sync(0xffffffffu, R.wk, j & 15);
+                if (idx < items) {
+                    const double2 ab = __ldg(reinterpret_cast<const double2*>(P) + pi);
+                    const double cc = 0.5 * (ab.x + ab.y), h = 0.5 * (ab.y - ab.x);
+                    const double tn = __dadd_rn(cc, __dmul_rn(h, xj));
+                    if (!(fast && greek_sums<BATES, true>(C, r, lambda, tn, h * wj, sum))) {
+                        double g[7];
+                        greek_sums_slow<BATES>(C, r, lambda, tn, h * wj, g);
+#pragma unroll
+                        for (int k = 0; k < 7; ++k) sum[k] += g[k];
+                    }
+                }
+            }
+            bool finite = true;
+#pragma unroll
+            for (int k = 0; k < 7; ++k) {
+                acc[k] = warp_sum(sum[k]);
+                finite = finite && isfinite(acc[k]);
+            }
+            if (finite || !fast) break;  // else each node again, dropping the terms that are not finite
+        }
         if (lane == 0) {
             double* out = B.part + w * 7;
 #pragma unroll
@@ -418,8 +409,7 @@ int grad_grid(K kernel, size_t smem, unsigned long long need, int* grid) {
 size_t grad_backward_bytes(size_t n, int dim) {
     const size_t units = 2 * n, slots = units * kMaxChunks;
     return align_up(units * sizeof(uint32_t), 256) + align_up(units, 256) +
-           align_up(slots * sizeof(unsigned long long), 256) + align_up(slots * (dim + 2) * sizeof(double), 256) +
-           align_up(n * 2 * dim * sizeof(double), 256) + 256;
+           align_up(slots * sizeof(unsigned long long), 256) + align_up(slots * dim * sizeof(double), 256) + 256;
 }
 
 namespace {
@@ -435,9 +425,7 @@ BackScratch carve_back_scratch(void* base, size_t n, int dim) {
     B.work = reinterpret_cast<unsigned long long*>(p);
     p += align_up(slots * sizeof(unsigned long long), 256);
     B.part = reinterpret_cast<double*>(p);
-    p += align_up(slots * (dim + 2) * sizeof(double), 256);
-    B.normd = reinterpret_cast<double*>(p);
-    p += align_up(n * 2 * dim * sizeof(double), 256);
+    p += align_up(slots * dim * sizeof(double), 256);
     B.count = reinterpret_cast<unsigned long long*>(p);
     return B;
 }
@@ -485,7 +473,7 @@ int launch_grad_backward(int model, const ope_contract* con, size_t n, const int
 
 size_t greeks_analytic_workspace_bytes(size_t n) {
     return align_up(n * sizeof(double), 256) + price_scratch_bytes(n) + panel_sink_bytes(n, 1) +
-           grad_backward_bytes(n, 5);  // 5 + 2 = 7 sums per chunk
+           grad_backward_bytes(n, 7);  // 7 sums per chunk
 }
 
 int launch_greeks_analytic(int model, const ope_contract* con, size_t n, const double* params, double tol,
@@ -498,7 +486,7 @@ int launch_greeks_analytic(int model, const ope_contract* con, size_t n, const d
     p += price_scratch_bytes(n);
     const PanelSink sink = carve_panel_sink(p, n, 1, nullptr);
     p += panel_sink_bytes(n, 1);
-    const BackScratch B = carve_back_scratch(p, n, 5);
+    const BackScratch B = carve_back_scratch(p, n, 7);
     // 1. prices, the integrals I1, I2 (s.integ) and the final panel lists
     OPE_TRY(launch_price_persistent(model, con, n, nullptr, 1, nullptr, params, tol, price, s, st, nullptr, nullptr,
                                     &sink));

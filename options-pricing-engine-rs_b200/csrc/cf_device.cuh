@@ -369,6 +369,20 @@ __device__ __forceinline__ double exp_node(double x) {
     return fma(sc, q, sc);
 }
 
+// cos and sin of r + K from r and the table's (cos K, sin K).
+__device__ __forceinline__ void cis_tail(double r, double2 cs, double& re, double& im) {
+    const double w = __dmul_rn(r, r);
+    double a = fma(-0.00019840255845338106, w, 0.008333333322977338);
+    a = fma(a, w, -0.16666666666666413);
+    const double sr = fma(__dmul_rn(a, w), r, r);  // sin r
+    double b = fma(2.4800567189231515e-05, w, -0.00138888880610466);
+    b = fma(b, w, 0.04166666666656595);
+    b = fma(b, w, -0.5);
+    const double cm = __dmul_rn(b, w);  // cos r - 1
+    re = fma(-cs.y, sr, fma(cs.x, cm, cs.x));
+    im = fma(cs.x, sr, fma(cs.y, cm, cs.y));
+}
+
 // cos x and sin x, branch-free: x = k pi/32 + r, |r| <= pi/64, pi/32 split into
 // 21 bits and the rest, sin r and cos r - 1 from polynomials (3e-19 and 6e-19
 // absolute, node_math_coeffs.py), then the angle sum with the table's
@@ -382,16 +396,18 @@ __device__ __forceinline__ void cis_node(double x, double& re, double& im) {
     const double2 cs = __ldg(g_cis_tab + (k & 63));
     double r = fma(kd, -0.09817475080490112, x);
     r = fma(kd, -1.9619779915655082e-08, r);
-    const double w = __dmul_rn(r, r);
-    double a = fma(-0.00019840255845338106, w, 0.008333333322977338);
-    a = fma(a, w, -0.16666666666666413);
-    const double sr = fma(__dmul_rn(a, w), r, r);  // sin r
-    double b = fma(2.4800567189231515e-05, w, -0.00138888880610466);
-    b = fma(b, w, 0.04166666666656595);
-    b = fma(b, w, -0.5);
-    const double cm = __dmul_rn(b, w);  // cos r - 1
-    re = fma(-cs.y, sr, fma(cs.x, cm, cs.x));
-    im = fma(cs.x, sr, fma(cs.y, cm, cs.y));
+    cis_tail(r, cs, re, im);
+}
+
+// The same for x + a, x taken as exact and reduced before a is added.
+__device__ __forceinline__ void cis_node(double x, double a, double& re, double& im) {
+    const double t = fma(__dadd_rn(x, a), 10.185916357881302, kRound);
+    const int k = __double2loint(t);
+    const double kd = __dsub_rn(t, kRound);
+    const double2 cs = __ldg(g_cis_tab + (k & 63));
+    double r = fma(kd, -0.09817477042468103, x);
+    r = __dadd_rn(fma(kd, -3.827021247335479e-18, r), a);
+    cis_tail(r, cs, re, im);
 }
 
 // sin(x + a) w, branch-free, x taken as exact and reduced before a is added:
@@ -570,8 +586,9 @@ struct CfConsts {
     double hxr, nhrs, hzr0, hzr2, hzi1, t, kts, ktst, kts2, nhv0, rtl, z0re, z0im;
     double jr0, hs2, jmu, lt;
     int sgn_bit;
-    // raw values kept for the adjoint chain
-    double kappa, rs, sgn, phi_im, sig2, v0s, rt, x, lnm_re, lnm_im, mu_j, comp;
+    // kept for the adjoint
+    double rs, sgn, phi_im, sig2, v0, rt, x, comp;
+    double z0;  // z0re without the logarithm's constant
 };
 
 // stable_cf at a general complex phi, following heston.rs:113-127's operation
@@ -612,11 +629,10 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
                                                 bool bates, int which) {
     const double v0 = p[0], kappa = p[1], theta = p[2], sigma = p[3], rho = p[4];
     CfConsts C;
-    C.kappa = kappa;
     C.rs = rho * sigma;
     C.sig2 = sigma * sigma;
     C.kts = (kappa * theta) / (sigma * sigma);
-    C.v0s = v0 / (sigma * sigma);
+    C.v0 = v0;
     C.t = t;
     C.rt = r * t;
     C.x = log_cr(s / k);  // heston.rs:86, rounded as the platform libm rounds it
@@ -640,14 +656,12 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
         comp = exp(p[6] + (0.5 * p[7]) * p[7]) - 1.0;
     }
     C.lt = lt;
-    C.mu_j = mu_j;
     C.hs2 = hs2;
     C.comp = comp;
     C.jr0 = -C.phi_im * mu_j + hs2 * (C.phi_im * C.phi_im);
     C.jmu = mu_j - 2.0 * hs2 * C.phi_im;
     C.rtl = C.rt - lt * comp;
-    C.lnm_re = 0.0;
-    C.lnm_im = 0.0;
+    double lnm_re = 0.0, lnm_im = 0.0;
     if (which == 0) {
         // CF(-i) = e^{rT} in exact arithmetic (C = D = 0 there, jump factor 1),
         // and the reference's operation sequence reproduces that to the last
@@ -659,21 +673,22 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
         // sequence.  (The regular case skips two complex exponentials, three
         // complex divisions and two complex logarithms per P1 integral.)
         bool regular = xr > 1e-100 && xr < 1e100 && C.sig2 > 1e-100 && C.kts < 1e4 &&
-                       C.v0s * xr < 1e4 && fabs(C.rt) < 700.0 && t < 1e3;
+                       v0 / (sigma * sigma) * xr < 1e4 && fabs(C.rt) < 700.0 && t < 1e3;
         if (bates) regular = regular && fabs(p[6] + 0.5 * p[7] * p[7]) < 50.0 && fabs(lt) * (comp + 1.0) < 1e4;
         if (regular) {
-            C.lnm_re = -C.rt;
+            lnm_re = -C.rt;
         } else {
             const Cx phi_mi{0.0, -1.0};
             Cx m = stable_cf_ref(phi_mi, t, r, v0, kappa, theta, sigma, rho);
             if (bates) m = cmul(m, jump_cf_ref(phi_mi, t, p[5], p[6], p[7]));
             Cx lm = clog(m);
-            C.lnm_re = -lm.re;
-            C.lnm_im = -lm.im;
+            lnm_re = -lm.re;
+            lnm_im = -lm.im;
         }
     }
-    C.z0re = (-C.rt * C.phi_im + C.lnm_re) + fma(C.kts, 0.6931471805599453, lt * (C.phi_im * comp - 1.0));
-    C.z0im = C.lnm_im;
+    C.z0 = (-C.rt * C.phi_im + lnm_re) + lt * (C.phi_im * comp - 1.0);
+    C.z0re = fma(C.kts, 0.6931471805599453, C.z0);
+    C.z0im = lnm_im;
     return C;
 }
 

@@ -30,7 +30,7 @@ def _table(name):
 
 
 def _body(name):
-    body = SRC[SRC.index(f"void {name}(" if name == "cis_node" else f"double {name}("):]
+    body = SRC[SRC.index(f"void {name}(" if name == "cis_tail" else f"double {name}("):]
     return body[:body.index("\n}\n")]
 
 
@@ -46,7 +46,7 @@ def test_tables_are_what_their_generator_derives():
 
 def test_coefficients_match_their_generator():
     s, c = coeffs.cis_coefficients()
-    for name, want in (("exp_node", coeffs.exp_coefficients()), ("cis_node", s), ("cis_node", c),
+    for name, want in (("exp_node", coeffs.exp_coefficients()), ("cis_tail", s), ("cis_tail", c),
                        ("sin_node", coeffs.sin_coefficients()), ("log_ratio", coeffs.log_ratio_coefficients()),
                        ("arg_node", coeffs.arg_coefficients())):
         have = _floats(_body(name))
