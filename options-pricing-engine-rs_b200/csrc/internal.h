@@ -118,7 +118,7 @@ struct PriceScratch {
     unsigned long long* head;      // 1   (must be zero before launch; persistent only)
     uint32_t* order = nullptr;     // n   queue position -> contract
     uint32_t* bucket = nullptr;    // n   depth bucket of each contract
-    unsigned int* hist = nullptr;  // 2 x 64 bucket counts and fill counters
+    unsigned int* hist = nullptr;  // 2 x 64 bucket counts and fill counters, resident-block counters
     // run cache of the run kernel (optional; run_cache_bytes() bytes): without
     // it a launch takes one contract per unit whatever its shape asks
     void* runcache = nullptr;
@@ -149,10 +149,13 @@ struct LaunchShape {
     // contracts per unit: 1 = one contract per unit (k_price_persistent);
     // 2..32 = blocks of that many consecutive contracts per warp, runs of
     // equal (parameter set, expiry, rate) sharing a run cache (k_price_runs,
-    // input order); 0 = automatic: a call of 32,768 contracts or more probes
+    // input order); 0 = automatic: a large call (pricing.cu: worth_probing) probes
     // its contracts on the device and takes the run kernel when its runs
     // average 4 contracts or more
     int per_unit = 0;
+    // not from a tuned table: queue order and resident warps go by the call
+    // (pricing.cu: order_by_size, k_order_scatter)
+    bool by_size = true;
 };
 // Bytes of the run cache for the current device (every warp the run
 // kernel's grid can hold); 0 without a device.
@@ -187,9 +190,9 @@ struct PanelSink {
 size_t panel_sink_bytes(size_t n, int n_slots);  // panels + nbis for n contracts
 PanelSink carve_panel_sink(void* base, size_t n, int n_slots, const int32_t* slot);
 // sink (non-NULL): also store every priced integral's panel list there.
-// shape (non-NULL): this launch shape instead of price_shape(model, n); a
-// launch that stores panel lists (sink) or skips surfaces (surf_mask) always
-// uses 4 warps per block in input order.
+// shape (non-NULL): this launch shape instead of price_shape(model, n).  A
+// launch that skips surfaces (surf_mask) always uses 4 warps per block in
+// input order; one that stores panel lists (sink) never a tuned shape.
 int launch_price_persistent(int model, const ope_contract* con, size_t n, const int64_t* surf_offsets,
                             size_t n_surf, const int32_t* param_idx, const double* params, double tol, double* out,
                             const PriceScratch& s, cudaStream_t st, int32_t* nbis_out = nullptr,

@@ -42,6 +42,8 @@ namespace ope {
 
 namespace {
 constexpr int kOrderBuckets = 64;
+constexpr int kSmSlots = 256;  // resident-block counters, by %smid
+constexpr size_t kHistBytes = (2 * kOrderBuckets + kSmSlots) * sizeof(unsigned int);
 // Run cache entries per warp (panels of one run), and warps per SM it is
 // sized for (the 64-register budget holds at most 32).
 #ifndef OPE_RUN_CACHE_ENTRIES
@@ -49,21 +51,31 @@ constexpr int kOrderBuckets = 64;
 #endif
 constexpr int kRunCacheEntries = OPE_RUN_CACHE_ENTRIES;
 constexpr int kRunWarpsPerSm = 32;
-// Automatic launches (per_unit 0): calls of at least kRunsMinContracts
-// contracts probe for runs (k_run_probe), which picks kRunsMinPerUnit to
-// kRunsMaxPerUnit contracts per unit, or the per-contract kernel.
-constexpr size_t kRunsMinContracts = 32768;
+// Automatic launches (per_unit 0): calls large enough for kRunsMinPerUnit
+// contracts per unit (worth_probing) probe for runs (k_run_probe), which picks
+// kRunsMinPerUnit to kRunsMaxPerUnit contracts per unit, or the per-contract
+// kernel.
 constexpr int kRunsMinPerUnit = 4;
 constexpr int kRunsMaxPerUnit = 16;
 constexpr int kRunsUnitsPerWarp = 24;
 constexpr size_t kRunCacheWarpBytes = (size_t)kRunCacheEntries * (2 * 16 * sizeof(double) + sizeof(uint32_t));
+
+// Whether the run probe could choose the run kernel: blocks of
+// kRunsMinPerUnit contracts must leave every warp of its grid at least
+// kRunsUnitsPerWarp units (227,328 contracts on 148 SMs).  1 / 4 contracts per
+// unit: 177,518 Heston grid contracts 3.84 / 4.27 ms, 373,066 8.16 / 8.07.
+bool worth_probing(size_t n) {
+    int sms = 0;
+    if (current_device_sms(&sms) != OPE_OK) return false;
+    return 2 * n >= (size_t)kRunsMinPerUnit * kRunsUnitsPerWarp * kRunWarpsPerSm * (size_t)sms;
+}
 }
 
 // Layout: integ (2n doubles) | done (n) | head (256 B) | hist (2 x kOrderBuckets
-// counters, 512 B) | order (n) | bucket (n); done, head and hist are adjacent
-// so one memset clears them.
+// counters, then kSmSlots resident-block counters) | order (n) | bucket (n);
+// done, head and hist are adjacent so one memset clears them.
 size_t price_scratch_bytes(size_t n) {
-    return align_up(2 * n * sizeof(double), 256) + align_up(n * sizeof(unsigned int), 256) + 256 + 512 +
+    return align_up(2 * n * sizeof(double), 256) + align_up(n * sizeof(unsigned int), 256) + 256 + kHistBytes +
            2 * align_up(n * sizeof(uint32_t), 256);
 }
 
@@ -82,7 +94,7 @@ PriceScratch carve_price_scratch(void* base, size_t n, size_t run_bytes) {
 
 size_t price_run_bytes(int model, size_t n, size_t other_bytes) {
     const int pu = price_shape(model, n).per_unit;
-    if (!(pu > 1 || (pu == 0 && n >= kRunsMinContracts))) return 0;
+    if (!(pu > 1 || (pu == 0 && worth_probing(n)))) return 0;
     const size_t b = run_cache_bytes();
     // under a workspace limit the run cache is optional: without it the call
     // takes one contract per unit, with the same prices
@@ -110,7 +122,7 @@ PriceScratch carve_price_scratch(void* base, size_t n) {
     s.head = reinterpret_cast<unsigned long long*>(p);
     p += 256;
     s.hist = reinterpret_cast<unsigned int*>(p);
-    p += 512;
+    p += kHistBytes;
     s.order = reinterpret_cast<uint32_t*>(p);
     p += align_up(n * sizeof(uint32_t), 256);
     s.bucket = reinterpret_cast<uint32_t*>(p);
@@ -219,8 +231,24 @@ __global__ void __launch_bounds__(WARPS * 32, (BATES ? OPE_KERNEL_MINB_BATES : O
                        long long n_surf, const int32_t* __restrict__ param_idx, const int32_t* __restrict__ surf_mask,
                        const double* __restrict__ params, double tol, double* __restrict__ out, double* integ,
                        unsigned int* done, unsigned long long* head, int32_t* nbis_out, PanelSink sink,
-                       const uint32_t* __restrict__ order) {
+                       const uint32_t* __restrict__ order, unsigned int* on_sm, int per_sm) {
     extern __shared__ PanelStore smem_panels[];
+    if (order) {
+        // a deepest-first launch may want fewer blocks on each SM
+        // (k_order_scatter): those past the limit leave at once
+        const int cap = (int)(long long)__ldcg(head + 1);
+        if (cap != 0) {
+            __shared__ int s_leave;
+            if (threadIdx.x == 0) {
+                unsigned sm;
+                asm("mov.u32 %0, %%smid;" : "=r"(sm));
+                const int mine = (int)atomicAdd(on_sm + (sm & (kSmSlots - 1)), 1u);
+                s_leave = mine >= max(1, cap > 0 ? (cap + WARPS / 2) / WARPS : per_sm + cap / WARPS);
+            }
+            __syncthreads();
+            if (s_leave) return;
+        }
+    }
     // Per warp: the unit's integrand constants.  They are warp-uniform, so the
     // node evaluation reads them from shared memory (broadcast loads) and
     // leaves its registers to the per-lane values: at the 72-register cap
@@ -423,10 +451,10 @@ __global__ void __launch_bounds__(256) k_run_probe(const ope_contract* __restric
 // Spearman correlation of 0.9 on the benchmark batches (short expiries and
 // deep wings need the most panels); 8 buckets per doubling of 1 + key.
 __device__ __forceinline__ unsigned depth_bucket(const ope_contract* con, long long c, double v0) {
-    const double x = fabs(log(__ldg(&con[c].strike) / __ldg(&con[c].spot)));
-    const double key = x / sqrt(fmax(v0, 0.0) * __ldg(&con[c].expiry));
+    const float x = fabsf(__logf((float)(__ldg(&con[c].strike) / __ldg(&con[c].spot))));
+    const float key = x * rsqrtf((float)(fmax(v0, 0.0) * __ldg(&con[c].expiry)));
     if (!(key == key)) return kOrderBuckets - 1;  // NaN (e.g. 0/0): last
-    const int b = (int)fmin(8.0 * log2(1.0 + key), (double)(kOrderBuckets - 1));
+    const int b = (int)fminf(8.0f * __log2f(1.0f + key), (float)(kOrderBuckets - 1));
     return (unsigned)(kOrderBuckets - 1 - b);
 }
 
@@ -449,13 +477,36 @@ __global__ void __launch_bounds__(256) k_order_bucket(const ope_contract* __rest
         if (h[i]) atomicAdd(hist + i, h[i]);
 }
 
+// Expected bisections of a contract in depth bucket `b` (0: deepest), up to a
+// factor: over the benchmark layouts at tol 1e-8 and 1e-10 the means of the
+// buckets lie on 7 + 2.2 key^0.92 (times 0.65 at 1e-8) within a fifth, capped
+// at 199.
+__device__ __forceinline__ float depth_estimate(int b) {
+    const float key = exp2f(((float)(kOrderBuckets - 1 - b) + 0.5f) * 0.125f) - 1.0f;
+    return fminf(199.0f, 7.0f + 2.2f * __powf(key, 0.92f));
+}
+
 // Queue positions: each block forms the buckets' starting positions (an
 // exclusive prefix sum of the kOrderBuckets counts hist[0..64), one warp),
 // then each contract takes the next free slot of its bucket through the fill
 // counters hist[64..128) (the order inside a bucket is arbitrary, and
 // irrelevant to the prices).
+//
+// sms > 0: block 0 also leaves in head[1] how many warps of the pricing kernel
+// are to stay resident on each SM (0: all, negative: that many fewer).  A chain's step takes the longer the more warps
+// share its scheduler, so a call whose deepest chain is long against its work
+// is done sooner with fewer resident warps.  With q = (expected steps of the
+// call per SM) / (expected steps of its deepest bucket), w warps per SM are
+// balanced (chain as long as the work) at w = q: 8 to 24 warps per SM by q up to
+// 52, one block less than resident up to 104, all above.  Measured on wings,
+// deepest-first with the best of 1-8 blocks / all blocks, ms (q): Bates 4,096
+// contracts 0.315 / 0.376 (7), 8,192 0.397 / 0.423 (14), 16,384 0.654 / 0.723
+// (29), 32,768 1.141 / 1.221 (57), 65,536 2.270 / 2.270 (114); Heston grids of
+// 22,654 contracts 0.524 / 0.551.  Input order and all blocks: 0.398, 0.506,
+// 0.822, 1.294, 2.435; 0.594.
 __global__ void __launch_bounds__(256) k_order_scatter(long long n, const uint32_t* __restrict__ bucket,
-                                                       unsigned int* hist, uint32_t* __restrict__ order) {
+                                                       unsigned int* hist, uint32_t* __restrict__ order,
+                                                       unsigned long long* head, int sms) {
     __shared__ unsigned int start[kOrderBuckets];
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
@@ -468,6 +519,19 @@ __global__ void __launch_bounds__(256) k_order_scatter(long long n, const uint32
         }
         start[2 * lane] = incl - (a + b);
         start[2 * lane + 1] = incl - b;
+        if (blockIdx.x == 0 && sms > 0) {
+            const float ea = depth_estimate(2 * lane), eb = depth_estimate(2 * lane + 1);
+            float steps = 2.0f * ((float)a * ea + (float)b * eb);
+            float deepest = a ? ea : (b ? eb : 0.0f);
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                steps += __shfl_xor_sync(0xffffffffu, steps, d);
+                deepest = fmaxf(deepest, __shfl_xor_sync(0xffffffffu, deepest, d));
+            }
+            const float q = steps / (deepest * (float)sms);
+            const int warps = q < 52.0f ? min(24, max(8, (int)(1.1f * q))) : (q < 104.0f ? -4 : 0);
+            if (lane == 0) head[1] = (unsigned long long)(long long)warps;
+        }
     }
     __syncthreads();
     unsigned int* fill = hist + kOrderBuckets;
@@ -475,6 +539,19 @@ __global__ void __launch_bounds__(256) k_order_scatter(long long n, const uint32
         const uint32_t b = bucket[c];
         order[start[b] + atomicAdd(fill + b, 1u)] = (uint32_t)c;
     }
+}
+
+// Whether an automatic launch takes its contracts deepest-first: calls of
+// several surfaces with 16 to 2,400 contracts per SM.  Below, the order's two
+// launches cost more than the tail it removes (the deepest chains, up to 199
+// bisections, starting last); above, the tail no longer shows (524,288 Bates
+// wing contracts: 18.24 / 18.23 ms with and without).  One surface under one
+// parameter set keeps input order: its chains are of a length.
+constexpr size_t kOrderMinPerSm = 16, kOrderMaxPerSm = 2400;
+bool order_by_size(size_t n, size_t n_surf, const int32_t* param_idx) {
+    int sms = 0;
+    if (n_surf <= 1 || param_idx || current_device_sms(&sms) != OPE_OK) return false;
+    return n >= kOrderMinPerSm * sms && n < kOrderMaxPerSm * sms;
 }
 
 template <class K>
@@ -491,16 +568,18 @@ template <bool BATES, bool SAVE, int WARPS>
 int launch_impl(const ope_contract* con, size_t n, const int64_t* surf_offsets, size_t n_surf,
                 const int32_t* param_idx, const double* params, double tol, double* out, const PriceScratch& s,
                 cudaStream_t st, int32_t* nbis_out, const int32_t* surf_mask, const PanelSink& sink,
-                const uint32_t* order, double occupancy) {
+                const uint32_t* order, const LaunchShape& sh) {
     const int threads = WARPS * 32;
     const size_t smem = WARPS * sizeof(PanelStore);
     int grid = 0;
-    OPE_TRY(persistent_grid(k_price_persistent<BATES, SAVE, WARPS>, threads, smem, occupancy, &grid));
+    OPE_TRY(persistent_grid(k_price_persistent<BATES, SAVE, WARPS>, threads, smem, sh.occupancy, &grid));
     const unsigned long long need = (2ull * n + WARPS - 1) / WARPS;
     grid = (int)std::min<unsigned long long>((unsigned long long)grid, need);
+    int sms = 0;
+    OPE_TRY(current_device_sms(&sms));
     k_price_persistent<BATES, SAVE, WARPS><<<grid, threads, smem, st>>>(
         con, (long long)n, surf_offsets, (long long)n_surf, param_idx, surf_mask, params, tol, out, s.integ, s.done,
-        s.head, nbis_out, sink, order);
+        s.head, nbis_out, sink, order, s.hist + 2 * kOrderBuckets, grid / sms);
     OPE_CHECK(cudaGetLastError());
     return OPE_OK;
 }
@@ -545,27 +624,27 @@ int launch_runs(const ope_contract* con, size_t n, const int64_t* surf_offsets, 
 }
 
 template <bool BATES>
-int launch_plain(int warps, const ope_contract* con, size_t n, const int64_t* surf_offsets, size_t n_surf,
+int launch_plain(const LaunchShape& sh, const ope_contract* con, size_t n, const int64_t* surf_offsets, size_t n_surf,
                  const int32_t* param_idx, const double* params, double tol, double* out, const PriceScratch& s,
-                 cudaStream_t st, int32_t* nbis_out, const uint32_t* order, double occupancy) {
+                 cudaStream_t st, int32_t* nbis_out, const uint32_t* order) {
     const PanelSink none{nullptr, nullptr, nullptr, 1};
-    switch (warps) {
+    switch (sh.warps) {
         case 1:
             return launch_impl<BATES, false, 1>(con, n, surf_offsets, n_surf, param_idx, params, tol, out, s, st,
-                                                nbis_out, nullptr, none, order, occupancy);
+                                                nbis_out, nullptr, none, order, sh);
         case 2:
             return launch_impl<BATES, false, 2>(con, n, surf_offsets, n_surf, param_idx, params, tol, out, s, st,
-                                                nbis_out, nullptr, none, order, occupancy);
+                                                nbis_out, nullptr, none, order, sh);
         default:
             return launch_impl<BATES, false, 4>(con, n, surf_offsets, n_surf, param_idx, params, tol, out, s, st,
-                                                nbis_out, nullptr, none, order, occupancy);
+                                                nbis_out, nullptr, none, order, sh);
     }
 }
 
 // Deepest-first queue order of the n contracts into s.order (s.hist, zeroed
-// by the caller, and s.bucket as scratch).
+// by the caller, and s.bucket as scratch); limit: also the pricing grid's limit.
 int build_order(int model, const ope_contract* con, size_t n, const int64_t* surf_offsets, size_t n_surf,
-                const int32_t* param_idx, const double* params, const PriceScratch& s, cudaStream_t st) {
+                const int32_t* param_idx, const double* params, const PriceScratch& s, cudaStream_t st, bool limit) {
     int sms = 0;
     OPE_TRY(current_device_sms(&sms));
     const long long want = (long long)((n + 255) / 256);
@@ -573,7 +652,7 @@ int build_order(int model, const ope_contract* con, size_t n, const int64_t* sur
     k_order_bucket<<<blocks, 256, 0, st>>>(con, (long long)n, surf_offsets, (long long)n_surf, param_idx, params,
                                            param_stride(model), s.bucket, s.hist);
     OPE_CHECK(cudaGetLastError());
-    k_order_scatter<<<blocks, 256, 0, st>>>((long long)n, s.bucket, s.hist, s.order);
+    k_order_scatter<<<blocks, 256, 0, st>>>((long long)n, s.bucket, s.hist, s.order, s.head, limit ? sms : 0);
     OPE_CHECK(cudaGetLastError());
     tctx().launches += 2;
     return OPE_OK;
@@ -606,15 +685,19 @@ int launch_price_persistent(int model, const ope_contract* con, size_t n, const 
                             const PanelSink* sink, const LaunchShape* shape) {
     if (n == 0) return OPE_OK;
     const bool bates = model == OPE_MODEL_BATES;
-    // stored panel lists and skipped surfaces keep the fixed shape (4 warps,
-    // input order); the allocation-free entry point has no order scratch
+    // skipped surfaces keep the fixed shape (4 warps, input order), stored
+    // panel lists the untuned one; the allocation-free entry point has no
+    // order scratch
     LaunchShape sh;
+    const bool can_order = s.order && n <= 0xffffffffull;
     if (!sink && !surf_mask) sh = shape ? *shape : price_shape(model, n);
-    if (!s.order || n > 0xffffffffull) sh.deepest_first = 0;
-    // contracts per unit: fixed (2..32), automatic (0: probe for runs in
-    // calls of kRunsMinContracts or more), or one per unit; the run kernel
-    // needs the run cache and serves plain launches only
-    if (!s.runcache || sink || surf_mask || sh.per_unit < 0 || (sh.per_unit == 0 && n < kRunsMinContracts))
+    const bool by_size = sh.by_size && !shape && !surf_mask && can_order && order_by_size(n, n_surf, param_idx);
+    if (by_size) sh.deepest_first = 1;
+    if (!can_order) sh.deepest_first = 0;
+    // contracts per unit: fixed (2..32), automatic (0: probe for runs where
+    // that could choose any), or one per unit; the run kernel needs the run
+    // cache and serves plain launches only
+    if (!s.runcache || sink || surf_mask || sh.per_unit < 0 || (sh.per_unit == 0 && !worth_probing(n)))
         sh.per_unit = 1;
     if (sh.per_unit > 32) sh.per_unit = 32;
     const bool probe = sh.per_unit == 0;
@@ -628,31 +711,29 @@ int launch_price_persistent(int model, const ope_contract* con, size_t n, const 
     const bool hist_adjacent = sh.deepest_first && reinterpret_cast<char*>(s.hist) == reinterpret_cast<char*>(s.head) + 256;
     const size_t head_bytes = 256;  // both queue heads and the probe's words
     if (adjacent) {
-        OPE_CHECK(cudaMemsetAsync(s.done, 0, done_bytes + (hist_adjacent ? 256 + 512 : head_bytes), st));
+        OPE_CHECK(cudaMemsetAsync(s.done, 0, done_bytes + (hist_adjacent ? 256 + kHistBytes : head_bytes), st));
     } else {
         OPE_CHECK(cudaMemsetAsync(s.done, 0, n * sizeof(unsigned int), st));
         OPE_CHECK(cudaMemsetAsync(s.head, 0, head_bytes, st));
     }
     if (sh.deepest_first && !(adjacent && hist_adjacent))
-        OPE_CHECK(cudaMemsetAsync(s.hist, 0, 2 * kOrderBuckets * sizeof(unsigned int), st));
+        OPE_CHECK(cudaMemsetAsync(s.hist, 0, kHistBytes, st));
     if (!sink && !surf_mask) {
         tctx().last_per_unit = sh.per_unit;
         tctx().last_probe = nullptr;
     }
     const uint32_t* order = nullptr;
     if (sh.deepest_first) {
-        OPE_TRY(build_order(model, con, n, surf_offsets, n_surf, param_idx, params, s, st));
+        OPE_TRY(build_order(model, con, n, surf_offsets, n_surf, param_idx, params, s, st, by_size));
         order = s.order;
     }
     if (sink) {
         OPE_TRY((bates ? launch_impl<true, true, 4> : launch_impl<false, true, 4>)(
-            con, n, surf_offsets, n_surf, param_idx, params, tol, out, s, st, nbis_out, surf_mask, *sink, nullptr,
-            1.0));
+            con, n, surf_offsets, n_surf, param_idx, params, tol, out, s, st, nbis_out, surf_mask, *sink, order, sh));
     } else if (surf_mask) {
         const PanelSink none{nullptr, nullptr, nullptr, 1};
         OPE_TRY((bates ? launch_impl<true, false, 4> : launch_impl<false, false, 4>)(
-            con, n, surf_offsets, n_surf, param_idx, params, tol, out, s, st, nbis_out, surf_mask, none, nullptr,
-            1.0));
+            con, n, surf_offsets, n_surf, param_idx, params, tol, out, s, st, nbis_out, surf_mask, none, nullptr, sh));
     } else if (sh.per_unit > 1) {
         OPE_TRY((bates ? launch_runs<true, 4> : launch_runs<false, 4>)(con, n, surf_offsets, n_surf, param_idx, params,
                                                                        tol, out, s, st, nbis_out, sh.per_unit,
@@ -670,16 +751,14 @@ int launch_price_persistent(int model, const ope_contract* con, size_t n, const 
         k_run_probe<<<pb, 256, 0, st>>>(con, (long long)n, surf_offsets, (long long)n_surf, param_idx, s.head,
                                         4ll * rgrid);
         OPE_CHECK(cudaGetLastError());
-        OPE_TRY((bates ? launch_plain<true> : launch_plain<false>)(sh.warps, con, n, surf_offsets, n_surf, param_idx,
-                                                                   params, tol, out, s, st, nbis_out, order,
-                                                                   sh.occupancy));
+        OPE_TRY((bates ? launch_plain<true> : launch_plain<false>)(sh, con, n, surf_offsets, n_surf, param_idx,
+                                                                   params, tol, out, s, st, nbis_out, order));
         OPE_TRY((bates ? launch_runs<true, 4> : launch_runs<false, 4>)(con, n, surf_offsets, n_surf, param_idx, params,
                                                                        tol, out, s, st, nbis_out, 0, sh.occupancy));
         tctx().launches += 2;
     } else {
-        OPE_TRY((bates ? launch_plain<true> : launch_plain<false>)(sh.warps, con, n, surf_offsets, n_surf, param_idx,
-                                                                   params, tol, out, s, st, nbis_out, order,
-                                                                   sh.occupancy));
+        OPE_TRY((bates ? launch_plain<true> : launch_plain<false>)(sh, con, n, surf_offsets, n_surf, param_idx,
+                                                                   params, tol, out, s, st, nbis_out, order));
     }
     tctx().launches += 1;
     return OPE_OK;

@@ -170,6 +170,7 @@ LaunchShape price_shape(int model, size_t n) {
     const auto it = g_tables.find(dev);
     if (it == g_tables.end() || !it->second.tuned[m]) return sh;
     const ope_tune_entry& e = it->second.e[m][class_of(n)];
+    sh.by_size = false;
     sh.warps = e.shape.warps_per_block;
     sh.deepest_first = e.shape.deepest_first;
     sh.occupancy = e.shape.occupancy;
