@@ -281,6 +281,64 @@ __global__ void __launch_bounds__(WARPS * 32, (BATES ? OPE_KERNEL_MINB_BATES : O
     }
 }
 
+// Small calls: one block of two warps per contract, its integrals one warp
+// each, combined through shared memory: no queue, no completion counters (and
+// so no memset before the launch), and the hardware's block order instead of
+// the persistent grid.  What bounds such a call is the latency of its deepest
+// chain, so the node evaluation gets 128 registers: 8 blocks per SM against 5 /
+// 10 / 16 (200 / 102 / 64 registers), us: 256 Bates wings 65.0 / 63.8 / 76.1 /
+// 85.0, 2,000 Bates wings 118 / 123 / 128 / 129, 8,192 deepest-first 314 (8),
+// 334 (10).
+// A parameter set the caller has at hand (`row`) arrives with the launch.
+struct ParamRow {
+    double p[8];
+};
+template <bool BATES, bool SAVE>
+__global__ void __launch_bounds__(64, 8)
+    k_price_small(const ope_contract* __restrict__ con, const int64_t* __restrict__ surf_off, long long n_surf,
+                  const int32_t* __restrict__ param_idx, const double* __restrict__ params, const ParamRow row,
+                  double tol, double* __restrict__ out, double* integ, int32_t* nbis_out, PanelSink sink,
+                  const uint32_t* __restrict__ order) {
+    __shared__ PanelStore s_panels[2];
+    __shared__ CfConsts s_consts[2];
+    __shared__ double s_integ[2];
+    const int which = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const LaneRule R = lane_rule(lane);
+    const long long c = order ? (long long)__ldg(order + blockIdx.x) : (long long)blockIdx.x;
+    const ContractView v = load_contract(con, c, lane);
+    long long s = 0;
+    double pl[8];
+    if (params) {
+        s = param_set(param_idx, surf_off, n_surf, c);
+        if (!param_idx && n_surf > 1 && !ope_check(s >= 0 && s < n_surf, CHK_SURFACE)) return;
+#pragma unroll
+        for (int i = 0; i < (BATES ? 8 : 5); ++i) pl[i] = __ldg(params + s * (BATES ? 8 : 5) + i);
+    } else {
+#pragma unroll
+        for (int i = 0; i < (BATES ? 8 : 5); ++i) pl[i] = row.p[i];
+    }
+    const CfConsts Cl = make_consts(v.s, v.k, v.t, v.r, pl, BATES, which);
+    if (lane == 0) s_consts[which] = Cl;
+    __syncwarp();
+    int nb;
+    const double I = gk_integrate_warp<BATES>(s_consts[which], tol, s_panels[which], lane, R, &nb);
+    if (SAVE) {
+        int slot = sink.slot ? __ldg(sink.slot + s) : 0;
+        if (!ope_check(slot >= 0 && slot < sink.n_slots, CHK_SLOT)) slot = 0;
+        const size_t idx = (size_t)(2 * c + which) * sink.n_slots + slot;
+        double2* dst = reinterpret_cast<double2*>(sink.panels + idx * (2 * kMaxPanels));
+        for (int i = lane; i <= nb; i += 32) dst[i] = s_panels[which].ab[i];
+        if (lane == 0) sink.nbis[idx] = nb;
+    }
+    if (lane == 0) {
+        if (nbis_out) nbis_out[2 * c + which] = nb;
+        if (SAVE) integ[2 * c + which] = I;
+        s_integ[which] = I;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) out[c] = finish_price(v.s, v.k, v.t, v.r, v.q, v.opt_type, s_integ[0], s_integ[1]);
+}
+
 // The run kernel: the queue hands out blocks of `per_unit` consecutive
 // contracts (unit 2b + which: integral `which` of block b), and one warp
 // integrates a block's contracts one after another.  A block splits into runs
@@ -554,6 +612,20 @@ bool order_by_size(size_t n, size_t n_surf, const int32_t* param_idx) {
     return n >= kOrderMinPerSm * sms && n < kOrderMaxPerSm * sms;
 }
 
+// Calls k_price_small takes instead of the persistent grid: up to 48 contracts
+// per SM in input order, 128 deepest-first (its blocks then start in that
+// order).  Kernel time, small / persistent, us: one Heston contract 13.9 / 17.3,
+// a 256-contract Heston surface 20.8 / 25.7, 2,048 Bates wings 125 / 169,
+// a 7,680-contract Heston surface 108.6 / 108.3, 12,800 164 / 158; deepest-first
+// (with the residency limit / here, order kernels included): Bates wings 4,096
+// 313 / 264, 8,192 391 / 314, 16,384 699 / 659, 22,654 Heston grid contracts
+// 530 / 527.
+constexpr size_t kSmallPerSm = 48, kSmallOrderedPerSm = 128;
+bool is_small(size_t n, bool ordered) {
+    int sms = 0;
+    return current_device_sms(&sms) == OPE_OK && n <= (ordered ? kSmallOrderedPerSm : kSmallPerSm) * (size_t)sms;
+}
+
 template <class K>
 int persistent_grid(K kernel, int threads, size_t smem, double occupancy, int* grid) {
     int per_sm = 0, sms = 0;
@@ -581,6 +653,20 @@ int launch_impl(const ope_contract* con, size_t n, const int64_t* surf_offsets, 
         con, (long long)n, surf_offsets, (long long)n_surf, param_idx, surf_mask, params, tol, out, s.integ, s.done,
         s.head, nbis_out, sink, order, s.hist + 2 * kOrderBuckets, grid / sms);
     OPE_CHECK(cudaGetLastError());
+    return OPE_OK;
+}
+
+template <bool BATES, bool SAVE>
+int launch_small(const ope_contract* con, size_t n, const int64_t* surf_offsets, size_t n_surf,
+                 const int32_t* param_idx, const double* params, const double* row, double tol, double* out,
+                 double* integ, cudaStream_t st, int32_t* nbis_out, const PanelSink& sink, const uint32_t* order) {
+    ParamRow r{};
+    if (row) std::copy(row, row + (BATES ? 8 : 5), r.p);
+    k_price_small<BATES, SAVE><<<(unsigned)n, 64, 0, st>>>(con, surf_offsets, (long long)n_surf, param_idx,
+                                                            row ? nullptr : params, r, tol, out, integ, nbis_out, sink,
+                                                            order);
+    OPE_CHECK(cudaGetLastError());
+    tctx().launches += 1;
     return OPE_OK;
 }
 
@@ -676,6 +762,8 @@ int prepare_price_kernels() {
     const size_t smem = 4 * sizeof(PanelStore);
     OPE_TRY(persistent_grid(k_price_persistent<false, false, 4>, threads, smem, 1.0, &grid));
     OPE_TRY(persistent_grid(k_price_persistent<true, false, 4>, threads, smem, 1.0, &grid));
+    OPE_TRY(persistent_grid(k_price_small<false, false>, 64, 0, 1.0, &grid));
+    OPE_TRY(persistent_grid(k_price_small<true, false>, 64, 0, 1.0, &grid));
     return OPE_OK;
 }
 
@@ -704,28 +792,39 @@ int launch_price_persistent(int model, const ope_contract* con, size_t n, const 
     if (sh.per_unit > 1) sh.deepest_first = 0;
     if (sh.warps != 1 && sh.warps != 2) sh.warps = 4;
     if (!(sh.occupancy > 0.0 && sh.occupancy <= 1.0)) sh.occupancy = 1.0;
+    if (!sink && !surf_mask) {
+        tctx().last_per_unit = sh.per_unit;
+        tctx().last_probe = nullptr;
+    }
+    const bool small = is_small(n, by_size) && !surf_mask && sh.per_unit == 1 && sh.warps == 4 &&
+                       sh.deepest_first == (int)by_size && sh.occupancy == 1.0 && tctx().grid_fraction == 1.0;
     // completion counters, queue head and (for a deepest-first order) the
     // bucket counters start at zero: one memset where they are adjacent
     const size_t done_bytes = align_up(n * sizeof(unsigned int), 256);
     const bool adjacent = reinterpret_cast<char*>(s.head) == reinterpret_cast<char*>(s.done) + done_bytes;
     const bool hist_adjacent = sh.deepest_first && reinterpret_cast<char*>(s.hist) == reinterpret_cast<char*>(s.head) + 256;
     const size_t head_bytes = 256;  // both queue heads and the probe's words
-    if (adjacent) {
-        OPE_CHECK(cudaMemsetAsync(s.done, 0, done_bytes + (hist_adjacent ? 256 + kHistBytes : head_bytes), st));
-    } else {
-        OPE_CHECK(cudaMemsetAsync(s.done, 0, n * sizeof(unsigned int), st));
-        OPE_CHECK(cudaMemsetAsync(s.head, 0, head_bytes, st));
+    if (!small) {
+        if (adjacent) {
+            OPE_CHECK(cudaMemsetAsync(s.done, 0, done_bytes + (hist_adjacent ? 256 + kHistBytes : head_bytes), st));
+        } else {
+            OPE_CHECK(cudaMemsetAsync(s.done, 0, n * sizeof(unsigned int), st));
+            OPE_CHECK(cudaMemsetAsync(s.head, 0, head_bytes, st));
+        }
     }
-    if (sh.deepest_first && !(adjacent && hist_adjacent))
+    if (sh.deepest_first && (small || !(adjacent && hist_adjacent)))
         OPE_CHECK(cudaMemsetAsync(s.hist, 0, kHistBytes, st));
-    if (!sink && !surf_mask) {
-        tctx().last_per_unit = sh.per_unit;
-        tctx().last_probe = nullptr;
-    }
     const uint32_t* order = nullptr;
     if (sh.deepest_first) {
-        OPE_TRY(build_order(model, con, n, surf_offsets, n_surf, param_idx, params, s, st, by_size));
+        OPE_TRY(build_order(model, con, n, surf_offsets, n_surf, param_idx, params, s, st, by_size && !small));
         order = s.order;
+    }
+    if (small) {
+        const PanelSink none{nullptr, nullptr, nullptr, 1};
+        return (sink ? (bates ? launch_small<true, true> : launch_small<false, true>)
+                     : (bates ? launch_small<true, false> : launch_small<false, false>))(
+            con, n, surf_offsets, n_surf, param_idx, params, nullptr, tol, out, s.integ, st, nbis_out,
+            sink ? *sink : none, order);
     }
     if (sink) {
         OPE_TRY((bates ? launch_impl<true, true, 4> : launch_impl<false, true, 4>)(
