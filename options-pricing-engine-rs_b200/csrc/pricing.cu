@@ -47,7 +47,7 @@ constexpr size_t kHistBytes = (2 * kOrderBuckets + kSmSlots) * sizeof(unsigned i
 // Run cache entries per warp (panels of one run), and warps per SM it is
 // sized for (the 64-register budget holds at most 32).
 #ifndef OPE_RUN_CACHE_ENTRIES
-#define OPE_RUN_CACHE_ENTRIES 128
+#define OPE_RUN_CACHE_ENTRIES kRunEntries
 #endif
 constexpr int kRunCacheEntries = OPE_RUN_CACHE_ENTRIES;
 constexpr int kRunWarpsPerSm = 32;
@@ -58,7 +58,8 @@ constexpr int kRunWarpsPerSm = 32;
 constexpr int kRunsMinPerUnit = 4;
 constexpr int kRunsMaxPerUnit = 16;
 constexpr int kRunsUnitsPerWarp = 24;
-constexpr size_t kRunCacheWarpBytes = (size_t)kRunCacheEntries * (2 * 16 * sizeof(double) + sizeof(uint32_t));
+constexpr size_t kRunCacheWarpBytes = (size_t)kRunCacheEntries * 2 * 16 * sizeof(double);
+constexpr size_t kRunSharedBytes = (kMaxPanels + kRunEntries + 15) / 16 * 16;  // per warp: slots, child links
 
 // Whether the run probe could choose the run kernel: blocks of
 // kRunsMinPerUnit contracts must leave every warp of its grid at least
@@ -350,8 +351,7 @@ __global__ void __launch_bounds__(64, 8)
 // reaches across blocks; contracts alone in their run are integrated
 // uncached.  Prices are bit-identical to k_price_persistent's.
 struct RunCacheMem {
-    double* vals;     // per warp of the grid: [2][cap][16] (w, a)
-    uint32_t* child;  // per warp of the grid: [cap]
+    double* vals;  // per warp of the grid: [2][cap][16] (w, a)
     int cap;
 };
 
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(WARPS * 32, OPE_RUNS_MINB * 4 / WARPS)
                  long long n_surf, const int32_t* __restrict__ param_idx, const double* __restrict__ params,
                  double tol, double* __restrict__ out, double* integ, unsigned int* done, unsigned long long* head,
                  int32_t* nbis_out, int per_unit_arg, RunCacheMem mem) {
-    extern __shared__ PanelStore smem_panels[];  // [WARPS], then the entry slots [WARPS][kMaxPanels]
+    extern __shared__ PanelStore smem_panels[];  // [WARPS], then the warps' kRunSharedBytes
     __shared__ CfConsts s_consts[WARPS];
     const unsigned FULL = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -372,8 +372,8 @@ __global__ void __launch_bounds__(WARPS * 32, OPE_RUNS_MINB * 4 / WARPS)
     rc.cap = mem.cap;
     rc.w = mem.vals + gw * 2 * (size_t)mem.cap * 16;
     rc.a = rc.w + (size_t)mem.cap * 16;
-    rc.child = mem.child + gw * (size_t)mem.cap;
-    rc.slot = reinterpret_cast<uint16_t*>(smem_panels + WARPS) + warp * kMaxPanels;
+    rc.slot = reinterpret_cast<uint8_t*>(smem_panels + WARPS) + warp * kRunSharedBytes;
+    rc.child = rc.slot + kMaxPanels;
     rc.n_alloc = 0;
     rc.on = false;
     // contracts per unit: the launch's, or (0) the run probe's choice; with
@@ -676,7 +676,7 @@ int launch_small(const ope_contract* con, size_t n, const int64_t* surf_offsets,
 template <bool BATES, int WARPS>
 int runs_grid(size_t n, const PriceScratch& s, int per_unit, double occupancy, int* grid) {
     const int threads = WARPS * 32;
-    const size_t smem = WARPS * (sizeof(PanelStore) + kMaxPanels * sizeof(uint16_t));
+    const size_t smem = WARPS * (sizeof(PanelStore) + kRunSharedBytes);
     OPE_TRY(persistent_grid(k_price_runs<BATES, WARPS>, threads, smem, occupancy, grid));
     const int pu = per_unit > 0 ? per_unit : kRunsMinPerUnit;
     const unsigned long long blocks = ((unsigned long long)n + pu - 1) / pu;
@@ -693,15 +693,12 @@ int launch_runs(const ope_contract* con, size_t n, const int64_t* surf_offsets, 
                 const int32_t* param_idx, const double* params, double tol, double* out, const PriceScratch& s,
                 cudaStream_t st, int32_t* nbis_out, int per_unit, double occupancy) {
     const int threads = WARPS * 32;
-    const size_t smem = WARPS * (sizeof(PanelStore) + kMaxPanels * sizeof(uint16_t));
+    const size_t smem = WARPS * (sizeof(PanelStore) + kRunSharedBytes);
     int grid = 0;
     OPE_TRY((runs_grid<BATES, WARPS>(n, s, per_unit, occupancy, &grid)));
-    const size_t cache_warps = s.runcache_bytes / kRunCacheWarpBytes;
     RunCacheMem mem;
     mem.cap = kRunCacheEntries;
     mem.vals = static_cast<double*>(s.runcache);
-    mem.child = reinterpret_cast<uint32_t*>(static_cast<char*>(s.runcache) +
-                                            cache_warps * (size_t)kRunCacheEntries * 2 * 16 * sizeof(double));
     k_price_runs<BATES, WARPS><<<grid, threads, smem, st>>>(con, (long long)n, surf_offsets, (long long)n_surf,
                                                              param_idx, params, tol, out, s.integ, s.done,
                                                              s.head + 16, nbis_out, per_unit, mem);

@@ -11,7 +11,7 @@
 // warp, and is maintained exactly as the reference maintains its Vec:
 //   * argmax by f64::total_cmp with the LAST maximum winning ties (errors are
 //     non-negative, so their IEEE bit patterns compare as unsigned integers
-//     in total_cmp order; the warp maximum is three redux.sync steps);
+//     in total_cmp order, and so do their leading bits);
 //   * swap_remove of the chosen panel, then push(left), push(right);
 //   * total += kl + kr - kw; err += el + er - ew, in that association;
 //   * stop when err <= tol or 200 panels are live.
@@ -133,15 +133,15 @@ __device__ __forceinline__ double gk_sums(double f, const LaneRule& R) {
 // bit-identical with and without the cache.  An entry's w and a are one
 // 128-byte line each (15 nodes and a zero pad, written whole so that L2
 // never fetches the rest of a partly written line from DRAM).
-constexpr uint16_t kNoEntry = 0xffff;
-constexpr uint32_t kNoChildren = 0xffffffffu;
+constexpr int kRunEntries = 128;  // entries of one run's tree at most: an entry's number fits a byte
+constexpr uint8_t kNoEntry = 0xff;
 
 struct RunCacheWarp {
     double* w;          // [cap][16]: W = e^{Re Z} / ((1 - t) t), NaN at nodes that are not live
     double* a;          // [cap][16]: Im Z without the phase
-    uint32_t* child;    // [cap]: children's entries, left | right << 16 (kNoChildren: none yet)
-    uint16_t* slot;     // shared, [kMaxPanels]: entry of each live panel of the running integral
-    int cap;            // entries (<= 65535)
+    uint8_t* child;     // shared, [kRunEntries]: left child's entry, the right one's is the next (kNoEntry: none yet)
+    uint8_t* slot;      // shared, [kMaxPanels]: entry of each live panel of the running integral
+    int cap;            // entries (<= kRunEntries)
     int n_alloc;        // entries in use (warp-uniform; 0 at the start of a run)
     bool on;            // cache this integral's panels (warp-uniform)
 };
@@ -178,6 +178,24 @@ __device__ __forceinline__ void run_cache_discard(RunCacheWarp& rc, int lane) {
     rc.n_alloc = 0;
 }
 
+// The panel of largest error, the last of equals, by all 64 bits of the keys
+// (errors are non-negative, so their bits order as they do).
+static __device__ __noinline__ int argmax_exact(const PanelStore& L, int len, int lane) {
+    const unsigned FULL = 0xffffffffu;
+    unsigned long long best = 0ull;
+    int bi = -1;
+    for (int i = lane; i < len; i += 32) {
+        const unsigned long long kk = L.ekey[i];
+        if (kk >= best) { best = kk; bi = i; }
+    }
+    // high word, then low word among the lanes holding the top high word, then
+    // the largest index holding both
+    const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
+    const unsigned mh = __reduce_max_sync(FULL, hi);
+    const unsigned ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
+    return (int)__reduce_max_sync(FULL, (hi == mh && lo == ml) ? (unsigned)(bi + 1) : 0u) - 1;
+}
+
 // Step hooks of gk_integrate_warp.  The pricing kernels use NoTrace (empty
 // and inlined: no code); the QAG trace kernel (trace.cu) records every step.
 //   first(lane, f, k0, e0): the first panel [0, 1] (f: this lane's integrand
@@ -197,7 +215,10 @@ struct NoTrace {
 // the four words of a swap_remove move in one load and one store; with both
 // children's values in every lane and lane 0 writing the whole list, the
 // 262k-contract Bates batch took 10.17 ms instead of 9.79, the run kernel's
-// 1.46M-contract grids 32.4 ms instead of 27.2.
+// 1.46M-contract grids 32.4 ms instead of 27.2.  The argmax on 24 bits of each
+// error with its index (one maximum over the warp instead of three, no
+// selects), the first step without branches of its own, and the run cache's
+// links in shared memory: 9.27 -> 9.05 and 27.0 -> 24.7 ms.
 //
 // Returns the integral (in the lanes with bit 3 clear).  `nbis` receives the
 // number of bisections (loop iterations of heston.rs:200-210); the final
@@ -216,10 +237,15 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
     const unsigned FULL = 0xffffffffu;
     double total = 0.0, err = 0.0;
     int len = 0;
-    // panel under evaluation in this half-warp; first step: [0, 1] in both
-    // halves, the right half's result unused
-    double pa = 0.0, pb = 1.0, kw = 0.0, ew = 0.0;
+    // panel under evaluation in this half-warp; first step: [0, 1] on the left,
+    // an empty panel, which adds nothing, on the right
+    double pa = R.half ? 0.5 : 0.0, pb = R.half ? 0.5 : 1.0, kw = 0.0, ew = 0.0;
     char* const list = reinterpret_cast<char*>(&L);
+    // errors beyond the live panels read as 0 in the argmax
+#pragma unroll
+    for (int j = 0; j < (kMaxPanels + 31) / 32; ++j)
+        if (lane + 32 * j < kMaxPanels) L.ekey[lane + 32 * j] = 0ull;
+    __syncwarp();
     // cache mode of the step (warp-uniform): hit = read entries el_/er_,
     // put = evaluate and store into them; neither = evaluate uncached.  The
     // first step's panel [0, 1] is entry 0.
@@ -271,32 +297,26 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
         const double v = gk_sums(f, R);
         const double e = __dmul_rn(fabs(__dsub_rn(v, __shfl_xor_sync(FULL, v, 8))), h), k = __dmul_rn(v, h);
         const double ex = __shfl_xor_sync(FULL, e, 16), kx = __shfl_xor_sync(FULL, k, 16);
-        const bool first = len == 0;
-        if (first) {
-            total = k;
-            err = e;
+        total = __dadd_rn(total, __dsub_rn(__dadd_rn(k, kx), kw));
+        err = __dadd_rn(err, __dsub_rn(__dadd_rn(e, ex), ew));
+        if (len == 0) {
             tr.first(lane, R.half ? 0.0 : f, k, e);
         } else {
-            total = __dadd_rn(total, __dsub_rn(__dadd_rn(k, kx), kw));
-            err = __dadd_rn(err, __dsub_rn(__dadd_rn(e, ex), ew));
             tr.step(len, lane, f, pa, pb, ew, k, e, kx, ex, err, total);
         }
         // push(left) over the list's last slot (its panel was bisected, or
-        // moved to the bisected one's slot below), push(right) behind it
-        if ((lane & 15) == 0 && !(first && R.half)) {
-            const int at = first ? 0 : len - 1 + R.half;
+        // moved to the bisected one's slot below), push(right) behind it (the
+        // first step's empty right panel is overwritten by the second's)
+        if ((lane & 15) == 0) {
+            const int at = max(len - 1, 0) + R.half;
             L.ekey[at] = (unsigned long long)__double_as_longlong(e);
             L.k[at] = k;
             L.ab[at] = make_double2(pa, pb);
             if (CACHED && rc->on) {
-                const int own = R.half ? er_ : el_;
-                rc->slot[at] = (uint16_t)own;
+                rc->slot[at] = (uint8_t)(R.half ? er_ : el_);
                 if (put) {
-                    rc->child[own] = kNoChildren;
-                    if (!first && !R.half) rc->child[sw_] = (uint32_t)el_ | ((uint32_t)er_ << 16);
-                } else if (hit && !first) {
-                    // the child's own child word, read when it is bisected
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(rc->child + own));
+                    if (len > 0 || R.half == 0) rc->child[R.half ? er_ : el_] = kNoEntry;
+                    if (len > 0 && R.half == 0) rc->child[sw_] = (uint8_t)el_;
                 }
             }
         }
@@ -304,32 +324,32 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
         __syncwarp();
         if (!(err > tol && len < kMaxPanels)) break;
         if (!ope_check(len < kMaxPanels, CHK_PANEL_COUNT)) break;
-        // argmax over the live list, last maximum wins (Iterator::max_by);
-        // chunks of 32 entries, stopping (warp-uniformly) after the last one in use
-        unsigned long long best = 0ull;
-        int bi = -1;
-#pragma unroll
-        for (int j = 0; j < (kMaxPanels + 31) / 32; ++j) {
-            if (32 * j >= len) break;
-            const int i = lane + 32 * j;
-            if (i < len) {
-                const unsigned long long kk = L.ekey[i];
-                if (kk >= best) { best = kk; bi = i; }
-            }
-        }
-        // warp maximum of the 64-bit keys (high word, then low word among the
-        // lanes holding the top high word), then the largest index holding it
+        // argmax over the live list, last maximum wins (Iterator::max_by): the
+        // top 24 bits of each error (exponent and 13 bits; no sign) with its
+        // index below them, the largest two per lane over chunks of 32
+        // entries (stopping, warp-uniformly, after the last one in use), one
+        // warp maximum.  Only where another error shares the winner's 24 bits
+        // (vote) are the full 64 bits compared.
+        int bi;
         {
-            const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
-            const unsigned mh = __reduce_max_sync(FULL, hi);
-            const unsigned ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
-            const unsigned mi = __reduce_max_sync(FULL, (hi == mh && lo == ml) ? (unsigned)(bi + 1) : 0u);
-            best = ((unsigned long long)mh << 32) | ml;
-            bi = (int)mi - 1;
+            const unsigned* hi = reinterpret_cast<const unsigned*>(L.ekey) + 1;  // high words, 2 apart
+            unsigned best = ((hi[2 * lane] << 1) & ~255u) | (unsigned)lane, second = 0u;
+#pragma unroll
+            for (int j = 1; j < (kMaxPanels + 31) / 32; ++j) {
+                if (32 * j >= len) break;
+                if (32 * j + 31 < kMaxPanels || lane + 32 * j < kMaxPanels) {
+                    const unsigned p = ((hi[2 * lane + 64 * j] << 1) & ~255u) | (unsigned)(lane + 32 * j);
+                    second = max(second, min(best, p));
+                    best = max(best, p);
+                }
+            }
+            const unsigned top = __reduce_max_sync(FULL, best);
+            bi = (int)(top & 255u);
+            if (__any_sync(FULL, ((best == top ? second : best) ^ top) < 256u)) bi = argmax_exact(L, len, lane);
         }
         if (!ope_check(bi >= 0 && bi < len, CHK_PANEL_INDEX)) bi = 0;
         const int w = bi, last = len - 1;
-        ew = __longlong_as_double((long long)best);
+        ew = __longlong_as_double((long long)L.ekey[w]);
         kw = L.k[w];
         const double2 ab = L.ab[w];
         const double m = 0.5 * (ab.x + ab.y);
@@ -347,12 +367,12 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
             el_ = er_ = kNoEntry;
             if (sw_ != kNoEntry && !ope_check(sw_ < rc->n_alloc, CHK_RUN_ENTRY)) sw_ = kNoEntry;
             if (sw_ != kNoEntry) {
-                const uint32_t ch = rc->child[sw_];
-                if (ch != kNoChildren) {
+                const int ch = rc->child[sw_];
+                if (ch != kNoEntry) {
                     hit = true;
-                    el_ = (int)(ch & 0xffffu);
-                    er_ = (int)(ch >> 16);
-                    if (!ope_check(el_ < rc->n_alloc && er_ < rc->n_alloc, CHK_RUN_ENTRY)) {
+                    el_ = ch;
+                    er_ = ch + 1;
+                    if (!ope_check(er_ < rc->n_alloc, CHK_RUN_ENTRY)) {
                         hit = false;  // evaluate uncached
                         el_ = er_ = kNoEntry;
                         sw_ = kNoEntry;
@@ -368,7 +388,7 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
         __syncwarp();  // every lane has read entry w before it is overwritten
         // swap_remove: the last entry takes the bisected one's slot
         if (lane < 4) *reinterpret_cast<unsigned long long*>(list + (R.copy_at + w * R.copy_by)) = word;
-        if (CACHED && rc->on && lane == 0) rc->slot[w] = (uint16_t)moved;
+        if (CACHED && rc->on && lane == 0) rc->slot[w] = (uint8_t)moved;
     }
     *nbis = len - 1;
     return total;
