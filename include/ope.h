@@ -394,7 +394,7 @@ typedef struct {
                               * set with the same expiry and rate (the strikes of one expiry of a surface
                               * laid out expiry by expiry) evaluates the characteristic function once per
                               * panel for the whole run (4 warps, input order).  0 (the default):
-                              * automatic -- a large call (227,328 contracts or more on 148 SMs) counts its runs on the
+                              * automatic -- a large call (151,552 contracts or more on 148 SMs) counts its runs on the
                               * device and takes blocks of 16 when they average 4 contracts or more.
                               * Prices are bit-identical in every mode. */
     int32_t reserved;        /* 0 */

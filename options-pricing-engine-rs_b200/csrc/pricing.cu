@@ -57,18 +57,22 @@ constexpr int kRunWarpsPerSm = 32;
 // kernel.
 constexpr int kRunsMinPerUnit = 4;
 constexpr int kRunsMaxPerUnit = 16;
-constexpr int kRunsUnitsPerWarp = 24;
+// Units every warp of the run kernel's grid is to have at `pu` contracts per
+// unit, so that the tail of a queue of long units stays short.  1 / 4 / 8 / 16
+// contracts per unit on Heston grids, ms: 92,529 contracts 1.98 / 2.04 / 2.27 /
+// 2.88, 177,518 3.83 / 3.68 / 4.34 / 6.01, 373,066 8.13 / 6.87 / 7.31 / 8.58,
+// 510,832 11.02 / 9.06 / 9.05 / 10.00, 1,459,714 31.6 / 24.9 / 23.1 / 22.9.
+__host__ __device__ constexpr int runs_units_per_warp(int pu) { return pu < 8 ? 16 : 28; }
 constexpr size_t kRunCacheWarpBytes = (size_t)kRunCacheEntries * 2 * 16 * sizeof(double);
-constexpr size_t kRunSharedBytes = (kMaxPanels + kRunEntries + 15) / 16 * 16;  // per warp: slots, child links
+constexpr size_t kRunSharedBytes = (kMaxPanels + kRunLinks + 15) / 16 * 16;  // per warp: slots, child links
 
 // Whether the run probe could choose the run kernel: blocks of
-// kRunsMinPerUnit contracts must leave every warp of its grid at least
-// kRunsUnitsPerWarp units (227,328 contracts on 148 SMs).  1 / 4 contracts per
-// unit: 177,518 Heston grid contracts 3.84 / 4.27 ms, 373,066 8.16 / 8.07.
+// kRunsMinPerUnit contracts must leave every warp of its grid its units
+// (151,552 contracts on 148 SMs).
 bool worth_probing(size_t n) {
     int sms = 0;
     if (current_device_sms(&sms) != OPE_OK) return false;
-    return 2 * n >= (size_t)kRunsMinPerUnit * kRunsUnitsPerWarp * kRunWarpsPerSm * (size_t)sms;
+    return 2 * n >= (size_t)kRunsMinPerUnit * runs_units_per_warp(kRunsMinPerUnit) * kRunWarpsPerSm * (size_t)sms;
 }
 }
 
@@ -344,14 +348,20 @@ __global__ void __launch_bounds__(64, 8)
 // contracts (unit 2b + which: integral `which` of block b), and one warp
 // integrates a block's contracts one after another.  A block splits into runs
 // -- maximal stretches of contracts with the same parameter set, expiry and
-// rate, whose integrands differ only in the phase u ln(S/K) -- and each run of
-// two or more contracts shares one run cache (quadrature.cuh), so a surface
-// laid out expiry by expiry evaluates the characteristic function once per
-// panel and expiry instead of once per panel and strike.  A run never
-// reaches across blocks; contracts alone in their run are integrated
-// uncached.  Prices are bit-identical to k_price_persistent's.
+// rate, whose integrands differ only in the phase u ln(S/K) -- and each run
+// shares one run cache (quadrature.cuh), so a surface laid out expiry by
+// expiry evaluates the characteristic function once per panel and expiry
+// instead of once per panel and strike.  A run never reaches across blocks.
+// Prices are bit-identical to k_price_persistent's.
+//
+// What bounds it: issue slots (77 % used), most of them the step's bookkeeping
+// (344 instructions per step, of which 85 FP64).  Without a per-run switch, with
+// a node's (W, A) as one 16-byte word, a sentinel entry in place of branches and
+// the node evaluation inline again (out of line, a miss saved and restored the
+// loop's registers through local memory): 24.7 -> 23.3 ms on 1.46M Heston grid
+// contracts (23.9 ms out of line; inline at 7 / 6 blocks 28.9 / 23.9 ms).
 struct RunCacheMem {
-    double* vals;  // per warp of the grid: [2][cap][16] (w, a)
+    double2* vals;  // per warp of the grid: [cap][16] (w, a)
     int cap;
 };
 
@@ -370,12 +380,12 @@ __global__ void __launch_bounds__(WARPS * 32, OPE_RUNS_MINB * 4 / WARPS)
     const size_t gw = (size_t)blockIdx.x * WARPS + warp;
     RunCacheWarp rc;
     rc.cap = mem.cap;
-    rc.w = mem.vals + gw * 2 * (size_t)mem.cap * 16;
-    rc.a = rc.w + (size_t)mem.cap * 16;
+    rc.wa = mem.vals + gw * (size_t)mem.cap * 16;
     rc.slot = reinterpret_cast<uint8_t*>(smem_panels + WARPS) + warp * kRunSharedBytes;
     rc.child = rc.slot + kMaxPanels;
     rc.n_alloc = 0;
-    rc.on = false;
+    if (lane == 0) rc.child[kNoEntry] = (uint8_t)kNoEntry;
+    __syncwarp();
     // contracts per unit: the launch's, or (0) the run probe's choice; with
     // no choice (the probe kept the per-contract kernel) the queue is closed
     int per_unit = per_unit_arg;
@@ -409,10 +419,7 @@ __global__ void __launch_bounds__(WARPS * 32, OPE_RUNS_MINB * 4 / WARPS)
             const long long c = c0 + i;
             const long long s = __shfl_sync(FULL, ps, i);
             if ((starts >> i) & 1u) {
-                const unsigned later = i < 31 ? starts >> (i + 1) : 0u;
-                const int next = later ? i + __ffs((int)later) : cnt;
                 run_cache_discard(rc, lane);
-                rc.on = next - i >= 2 && rc.cap > 0;
             }
             if (!param_idx && n_surf > 1 && !ope_check(s >= 0 && s < n_surf, CHK_SURFACE)) continue;
             run_unit<BATES, false, true>(c, which, con, params + s * stride, tol, out, integ, done, nbis_out, none,
@@ -426,7 +433,7 @@ __global__ void __launch_bounds__(WARPS * 32, OPE_RUNS_MINB * 4 / WARPS)
 // expiry or rate) and, in its last block to finish, picks the contracts per
 // unit: the largest power of two up to 16 that is at most the sample's mean
 // run length and leaves every warp of the run kernel's grid (run_warps) at
-// least kRunsUnitsPerWarp units, so that the queue's tail stays short.
+// least runs_units_per_warp units.
 // Below kRunsMinPerUnit it keeps the per-contract kernel.  The sample: up to
 // kProbeChunks chunks of 32 consecutive contracts spread evenly over the
 // call, one warp each, every lane reading one contract's expiry and rate
@@ -493,7 +500,8 @@ __global__ void __launch_bounds__(256) k_run_probe(const ope_contract* __restric
             int pu = kRunsMaxPerUnit;
             while (pu >= kRunsMinPerUnit &&
                    (s_seen < (unsigned long long)pu * s_starts ||
-                    2ull * (unsigned long long)n < (unsigned long long)pu * kRunsUnitsPerWarp * (unsigned long long)run_warps))
+                    2ull * (unsigned long long)n <
+                        (unsigned long long)(pu * runs_units_per_warp(pu)) * (unsigned long long)run_warps))
                 pu >>= 1;
             const bool runs = pu >= kRunsMinPerUnit;
             head[25] = runs ? (unsigned long long)pu : 0ull;
@@ -698,7 +706,7 @@ int launch_runs(const ope_contract* con, size_t n, const int64_t* surf_offsets, 
     OPE_TRY((runs_grid<BATES, WARPS>(n, s, per_unit, occupancy, &grid)));
     RunCacheMem mem;
     mem.cap = kRunCacheEntries;
-    mem.vals = static_cast<double*>(s.runcache);
+    mem.vals = static_cast<double2*>(s.runcache);
     k_price_runs<BATES, WARPS><<<grid, threads, smem, st>>>(con, (long long)n, surf_offsets, (long long)n_surf,
                                                              param_idx, params, tol, out, s.integ, s.done,
                                                              s.head + 16, nbis_out, per_unit, mem);

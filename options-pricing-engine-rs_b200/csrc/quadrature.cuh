@@ -125,44 +125,25 @@ __device__ __forceinline__ double gk_sums(double f, const LaneRule& R) {
 // its entry (kNoEntry: not cached, nor are its descendants), so a bisection
 // finds its children's values with one load, without searching.  A contract
 // whose next panel is in the tree skips node_cf (the CF, its square root,
-// logarithm and exponentials) and pays only node_finish (its own phase and
-// one sin).  The tree lives in global memory (per warp: cap entries of 15
+// logarithm and exponentials) and pays only node_finish_w (its own phase and
+// one sine).  The tree lives in global memory (per warp: cap entries of 15
 // nodes x {W, A}); when it is full, further panels are evaluated
 // uncached.  The cached values are the ones node_cf's result gives (u is
 // recomputed from the node, bit for bit), so a contract's price is
-// bit-identical with and without the cache.  An entry's w and a are one
-// 128-byte line each (15 nodes and a zero pad, written whole so that L2
-// never fetches the rest of a partly written line from DRAM).
-constexpr int kRunEntries = 128;  // entries of one run's tree at most: an entry's number fits a byte
-constexpr uint8_t kNoEntry = 0xff;
+// bit-identical with and without the cache.  An entry is two whole
+// 128-byte lines (15 nodes and the pad lane's, so that L2 never fetches the
+// rest of a partly written line from DRAM).
+constexpr int kRunEntries = 127;    // entries of one run's tree at most
+constexpr int kNoEntry = 127;       // not cached; as an entry it has no children
+constexpr int kRunLinks = 128;
 
 struct RunCacheWarp {
-    double* w;          // [cap][16]: W = e^{Re Z} / ((1 - t) t), NaN at nodes that are not live
-    double* a;          // [cap][16]: Im Z without the phase
-    uint8_t* child;     // shared, [kRunEntries]: left child's entry, the right one's is the next (kNoEntry: none yet)
-    uint8_t* slot;      // shared, [kMaxPanels]: entry of each live panel of the running integral
-    int cap;            // entries (<= kRunEntries)
-    int n_alloc;        // entries in use (warp-uniform; 0 at the start of a run)
-    bool on;            // cache this integral's panels (warp-uniform)
+    double2* wa;     // [cap][16]: W = e^{Re Z} / ((1 - t) t), NaN at nodes that are not live, and Im Z without the phase
+    uint8_t* child;  // shared, [kRunLinks]: left child's entry, the right one's is the next (kNoEntry: none yet)
+    uint8_t* slot;   // shared, [kMaxPanels]: entry of each live panel of the running integral
+    int cap;         // entries (1..kRunEntries)
+    int n_alloc;     // entries in use (warp-uniform; 0 at the start of a run)
 };
-
-// node_cf as a real call, for the cached loop: a cache hit needs few
-// registers, and the call keeps the node evaluation's register demand (and
-// its spills) out of the hit path.
-// (Internal linkage, so that ptxas allocates its registers within the
-// calling kernel's budget.)
-// It returns the cached form: W with the liveness folded in (node_w_live),
-// A and u.
-namespace {
-struct NodeW {
-    double w, a, u;
-};
-template <bool BATES>
-__device__ __noinline__ NodeW node_cf_call(const CfConsts& C, double tn) {
-    const NodeCf n = node_cf<BATES>(C, tn);
-    return NodeW{node_w_live(tn, n), n.a, n.u};
-}
-}  // namespace
 
 // End of a run: its entries will be rewritten before they are read again, so
 // their lines are dropped from L2 without being written back to DRAM
@@ -170,10 +151,8 @@ __device__ __noinline__ NodeW node_cf_call(const CfConsts& C, double tn) {
 // costing DRAM bandwidth.  Warp-collective.
 __device__ __forceinline__ void run_cache_discard(RunCacheWarp& rc, int lane) {
     __syncwarp();
-    for (int j = lane; j < 2 * rc.n_alloc; j += 32) {
-        const double* line = j < rc.n_alloc ? rc.w + (size_t)j * 16 : rc.a + (size_t)(j - rc.n_alloc) * 16;
-        asm volatile("discard.global.L2 [%0], 128;" ::"l"(line) : "memory");
-    }
+    for (int j = lane; j < 2 * rc.n_alloc; j += 32)
+        asm volatile("discard.global.L2 [%0], 128;" ::"l"(rc.wa + (size_t)j * 8) : "memory");
     __syncwarp();
     rc.n_alloc = 0;
 }
@@ -250,16 +229,11 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
     // put = evaluate and store into them; neither = evaluate uncached.  The
     // first step's panel [0, 1] is entry 0.
     bool hit = false, put = false;
-    int el_ = kNoEntry, er_ = kNoEntry, sw_ = kNoEntry;  // sw_: entry of the bisected panel
-    if (CACHED && rc->on) {
-        if (rc->n_alloc > 0) {
-            hit = true;
-            el_ = er_ = 0;
-        } else if (rc->cap > 0) {
-            put = true;
-            el_ = 0;
-            rc->n_alloc = 1;
-        }
+    int el_ = 0, sw_ = kNoEntry;  // left child's entry (the right one's is the next), entry of the bisected panel
+    if (CACHED) {
+        hit = rc->n_alloc > 0;
+        put = !hit;
+        if (put) rc->n_alloc = 1;
     }
     while (true) {
         const double c = 0.5 * (pa + pb), h = 0.5 * (pb - pa);
@@ -268,28 +242,19 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
         // pad lanes 15 and 31 evaluate the panel's centre; their weights are 0.
         double nw, na, nu;
         if (CACHED && hit) {
-            const size_t i = (size_t)(R.half ? er_ : el_) * 16 + (lane & 15);
-            nw = __ldcg(rc->w + i);
-            na = __ldcg(rc->a + i);
+            // (the first step's right half reads the root's entry too)
+            const double2 wa = __ldcg(rc->wa + (el_ + (len > 0 ? R.half : 0)) * 16 + (lane & 15));
+            nw = wa.x;
+            na = wa.y;
             nu = node_u_of(tn);
         } else {
-            if (CACHED) {
-                const NodeW nc = node_cf_call<BATES>(C, tn);
-                nw = nc.w;
-                na = nc.a;
-                nu = nc.u;
-            } else {
-                const NodeCf nc = node_cf<BATES>(C, tn);
-                nw = node_w(nc);
-                na = nc.a;
-                nu = nc.u;
-            }
+            const NodeCf nc = node_cf<BATES>(C, tn);
+            nw = CACHED ? node_w_live(tn, nc) : node_w(nc);
+            na = nc.a;
+            nu = nc.u;
             // each half-warp writes its child's entry whole, pad lane included
-            if (CACHED && put && (len > 0 || R.half == 0)) {
-                const size_t i = (size_t)(R.half ? er_ : el_) * 16 + (lane & 15);
-                __stcg(rc->w + i, nw);
-                __stcg(rc->a + i, na);
-            }
+            if (CACHED && put && (len > 0 || R.half == 0))
+                __stcg(rc->wa + (el_ + R.half) * 16 + (lane & 15), make_double2(nw, na));
         }
         const double f = node_finish_w<CACHED>(C.x, tn, nw, na, nu);
         // K (in the lanes with bit 3 clear) and error of this half's child,
@@ -312,12 +277,13 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
             L.ekey[at] = (unsigned long long)__double_as_longlong(e);
             L.k[at] = k;
             L.ab[at] = make_double2(pa, pb);
-            if (CACHED && rc->on) {
-                rc->slot[at] = (uint8_t)(R.half ? er_ : el_);
-                if (put) {
-                    if (len > 0 || R.half == 0) rc->child[R.half ? er_ : el_] = kNoEntry;
-                    if (len > 0 && R.half == 0) rc->child[sw_] = (uint8_t)el_;
-                }
+            if (CACHED) {
+                // the children's entries, with no children of their own yet
+                // (a first step's right half leaves the root's alone)
+                const int own = el_ == kNoEntry ? kNoEntry : el_ + R.half;
+                rc->slot[at] = (uint8_t)own;
+                if (put && (len > 0 || R.half == 0)) rc->child[own] = (uint8_t)kNoEntry;
+                if (put && len > 0 && R.half == 0) rc->child[sw_] = (uint8_t)el_;
             }
         }
         ++len;
@@ -358,37 +324,28 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
         unsigned long long word = 0;
         if (lane < 4) word = *reinterpret_cast<const unsigned long long*>(list + (R.copy_at + last * R.copy_by));
         int moved = 0;
-        if (CACHED && rc->on) {
+        if (CACHED) {
             // the children of panel w: in the tree (hit), or new entries (put)
             // while the tree has room for both and w is in it
             sw_ = rc->slot[w];
             moved = rc->slot[last];
-            hit = put = false;
-            el_ = er_ = kNoEntry;
-            if (sw_ != kNoEntry && !ope_check(sw_ < rc->n_alloc, CHK_RUN_ENTRY)) sw_ = kNoEntry;
-            if (sw_ != kNoEntry) {
-                const int ch = rc->child[sw_];
-                if (ch != kNoEntry) {
-                    hit = true;
-                    el_ = ch;
-                    er_ = ch + 1;
-                    if (!ope_check(er_ < rc->n_alloc, CHK_RUN_ENTRY)) {
-                        hit = false;  // evaluate uncached
-                        el_ = er_ = kNoEntry;
-                        sw_ = kNoEntry;
-                    }
-                } else if (rc->n_alloc + 2 <= rc->cap) {
-                    put = true;
-                    el_ = rc->n_alloc;
-                    er_ = rc->n_alloc + 1;
-                    rc->n_alloc += 2;
-                }
+            if (!ope_check(sw_ < rc->n_alloc || sw_ == kNoEntry, CHK_RUN_ENTRY)) sw_ = kNoEntry;
+            el_ = rc->child[sw_];
+            hit = el_ != kNoEntry;
+            if (!ope_check(!hit || el_ + 1 < rc->n_alloc, CHK_RUN_ENTRY)) {
+                hit = false;  // evaluate uncached
+                el_ = sw_ = kNoEntry;
+            }
+            put = !hit && sw_ != kNoEntry && rc->n_alloc + 2 <= rc->cap;
+            if (put) {
+                el_ = rc->n_alloc;
+                rc->n_alloc += 2;
             }
         }
         __syncwarp();  // every lane has read entry w before it is overwritten
         // swap_remove: the last entry takes the bisected one's slot
         if (lane < 4) *reinterpret_cast<unsigned long long*>(list + (R.copy_at + w * R.copy_by)) = word;
-        if (CACHED && rc->on && lane == 0) rc->slot[w] = (uint8_t)moved;
+        if (CACHED && lane == 0) rc->slot[w] = (uint8_t)moved;
     }
     *nbis = len - 1;
     return total;
