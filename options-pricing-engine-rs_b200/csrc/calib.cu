@@ -86,6 +86,8 @@ struct LMDev {
     double* res;     // nq
     double* res_new; // nq
     double* jrow;    // nq x dim
+    double* iv;      // nq: implied vols at the current parameters' prices (negative: no solution)
+    double* iv_new;  // nq: the same at the trial prices
     unsigned int* counters;  // [0] active surfaces, [1] body passes
     const double* prior;     // ns x dim Tikhonov prior, or null
     const double* regw;      // ns regularisation weights
@@ -220,15 +222,18 @@ __global__ void k_lm_init(LMDev D, const double* p0) {
 }
 
 // IV residual of every quote whose surface is selected by `mask`
-// (calibration.rs:573-581): iv(model price) - iv_market, 0 if the solver fails.
-__global__ void k_lm_residuals(LMDev D, const int32_t* mask, const double* price, double* res) {
+// (calibration.rs:573-581): iv(model price) - iv_market, 0 if the solver fails;
+// the IV itself is kept for the Jacobian at these prices.
+__global__ void k_lm_residuals(LMDev D, const int32_t* mask, const double* price, double* res, double* ivs) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= D.nq) return;
     const int s = D.sidx[i];
     if (mask && mask[s] == 0) return;
     double iv;
     const IvC c = iv_contract(D.q[i]);
-    res[i] = implied_vol_d(c, price[i], &iv) ? iv - D.iv_mkt[i] : 0.0;
+    const bool ok = implied_vol_d(c, price[i], &iv);
+    res[i] = ok ? iv - D.iv_mkt[i] : 0.0;
+    ivs[i] = ok ? iv : -1.0;
 }
 
 // Jacobian rows at p for surfaces in jmask: d iv / d p = d price / d p / vega(iv)
@@ -238,11 +243,10 @@ __global__ void k_lm_jrows(LMDev D) {
     if (i >= D.nq) return;
     const int s = D.sidx[i];
     if (D.jmask[s] == 0) return;
-    const IvC c = iv_contract(D.q[i]);
-    double iv;
+    const double iv = D.iv[i];
     double scale = 0.0;
-    if (implied_vol_d(c, D.price[i], &iv)) {
-        const double vega = bsm_vega_d(c, iv);
+    if (iv > 0.0) {
+        const double vega = bsm_vega_d(iv_contract(D.q[i]), iv);
         if (fabs(vega) >= 1e-10) scale = 1.0 / vega;
     }
     for (int k = 0; k < D.dim; ++k) D.jrow[(size_t)i * D.dim + k] = D.pgrad[(size_t)i * D.dim + k] * scale;
@@ -364,6 +368,7 @@ __global__ void k_lm_accept(LMDev D) {
         for (int64_t i = D.off[s] + lane; i < D.off[s + 1]; i += 32) {
             D.res[i] = D.res_new[i];
             D.price[i] = D.price_trial[i];
+            D.iv[i] = D.iv_new[i];
         }
     if (lane != 0) return;
     const int dim = D.dim;
@@ -491,7 +496,7 @@ thread_local CalibGraph g_lm_graph;
 struct Layout {
     size_t total;
     size_t q, iv, w, off, sidx, st, pcur, ptrial, jmask, tmask, price, price_trial, jslot, pslot, pgrad, res, res_new,
-        jrow, counters, out, prior, regw, group, gbest, sink, bscr, scratch;
+        jrow, iv_cur, iv_new, counters, out, prior, regw, group, gbest, sink, bscr, scratch;
 };
 
 Layout layout(size_t nq, size_t ns, int dim) {
@@ -516,6 +521,8 @@ Layout layout(size_t nq, size_t ns, int dim) {
     L.res = take(nq * sizeof(double));
     L.res_new = take(nq * sizeof(double));
     L.jrow = take(nq * dim * sizeof(double));
+    L.iv_cur = take(nq * sizeof(double));
+    L.iv_new = take(nq * sizeof(double));
     L.counters = take(4 * sizeof(unsigned int));
     L.out = take(ns * sizeof(ope_calib_result));
     L.prior = take(ns * dim * sizeof(double));
@@ -552,6 +559,8 @@ LMDev make_dev(char* base, const Layout& L, int nq, int ns, int dim) {
     D.res = reinterpret_cast<double*>(base + L.res);
     D.res_new = reinterpret_cast<double*>(base + L.res_new);
     D.jrow = reinterpret_cast<double*>(base + L.jrow);
+    D.iv = reinterpret_cast<double*>(base + L.iv_cur);
+    D.iv_new = reinterpret_cast<double*>(base + L.iv_new);
     D.counters = reinterpret_cast<unsigned int*>(base + L.counters);
     D.prior = nullptr;
     D.regw = nullptr;
@@ -587,7 +596,7 @@ int enqueue_body(int model, const LMDev& D, char* base, const Layout& L, double 
     const PanelSink sink = pricing_sink(D, base, L);
     OPE_TRY(launch_price_persistent(model, D.q, D.nq, D.off, D.ns, nullptr, D.ptrial, tol, D.price_trial,
                                     carve_price_scratch(base + L.scratch, D.nq), st, nullptr, D.tmask, &sink));
-    k_lm_residuals<<<(D.nq + 127) / 128, 128, 0, st>>>(D, D.tmask, D.price_trial, D.res_new);
+    k_lm_residuals<<<(D.nq + 127) / 128, 128, 0, st>>>(D, D.tmask, D.price_trial, D.res_new, D.iv_new);
     OPE_CHECK(cudaGetLastError());
     k_lm_accept<<<warps_blocks, 128, 0, st>>>(D);
     OPE_CHECK(cudaGetLastError());
@@ -711,7 +720,7 @@ int calib_enqueue(int model, const ope_contract* quotes, const double* iv_market
     const PanelSink sink = pricing_sink(D, base, L);
     OPE_TRY(launch_price_persistent(model, D.q, nq, D.off, ns, nullptr, D.pcur, tol, D.price,
                                     carve_price_scratch(base + L.scratch, nq), st, nullptr, D.tmask, &sink));
-    k_lm_residuals<<<((int)nq + 127) / 128, 128, 0, st>>>(D, nullptr, D.price, D.res);
+    k_lm_residuals<<<((int)nq + 127) / 128, 128, 0, st>>>(D, nullptr, D.price, D.res, D.iv);
     OPE_CHECK(cudaGetLastError());
     k_lm_sse0<<<((int)ns * 32 + 127) / 128, 128, 0, st>>>(D);
     OPE_CHECK(cudaGetLastError());
@@ -833,10 +842,10 @@ int run_calib_jacobian(int model, const ope_contract* quotes, const double* iv_m
     const PanelSink sink = pricing_sink(D, base, L);
     OPE_TRY(launch_price_persistent(model, D.q, nq, D.off, ns, nullptr, D.pcur, tol, D.price,
                                     carve_price_scratch(base + L.scratch, nq), st, nullptr, nullptr, &sink));
-    OPE_TRY(launch_jac(model, D, base, L, st));
-    k_lm_residuals<<<((int)nq + 127) / 128, 128, 0, st>>>(D, nullptr, D.price, D.res);
+    k_lm_residuals<<<((int)nq + 127) / 128, 128, 0, st>>>(D, nullptr, D.price, D.res, D.iv);
     OPE_CHECK(cudaGetLastError());
     c.launches += 1;
+    OPE_TRY(launch_jac(model, D, base, L, st));
     OPE_CHECK(cudaMemcpyAsync(out_jac, D.jrow, nq * dim * sizeof(double), cudaMemcpyDeviceToHost, st));
     if (out_res) OPE_CHECK(cudaMemcpyAsync(out_res, D.res, nq * sizeof(double), cudaMemcpyDeviceToHost, st));
     OPE_CHECK(cudaStreamSynchronize(st));
