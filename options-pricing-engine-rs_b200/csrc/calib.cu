@@ -283,6 +283,24 @@ __device__ void surf_normal_eq(const LMDev& D, int s, int lane, double* jtj, dou
     }
 }
 
+// One Jacobian evaluation's set-up: each quote's surface (the s with off[s] <= i
+// < off[s + 1]), every surface selected, panel lists in slot 0.
+__global__ void k_jac_init(LMDev D) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < D.nq) {
+        int lo = 1, hi = D.ns;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (D.off[mid] > i) hi = mid; else lo = mid + 1;
+        }
+        const_cast<int32_t*>(D.sidx)[i] = lo - 1;
+    } else if (i - D.nq < D.ns) {
+        D.jmask[i - D.nq] = 1;
+        D.jslot[i - D.nq] = 0;
+        D.pslot[i - D.nq] = 0;
+    }
+}
+
 // One warp per surface: J'J, gradient test, damped step, bounds test.
 __global__ void k_lm_step(LMDev D) {
     const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -505,11 +523,11 @@ Layout layout(size_t nq, size_t ns, int dim) {
     auto take = [&](size_t bytes) { size_t at = o; o += align_up(bytes, 256); return at; };
     L.q = take(nq * sizeof(ope_contract));
     L.iv = take(nq * sizeof(double));
-    L.w = take(nq * sizeof(double));
     L.off = take((ns + 1) * sizeof(int64_t));
+    L.pcur = take(ns * dim * sizeof(double));
+    L.w = take(nq * sizeof(double));
     L.sidx = take(nq * sizeof(int32_t));
     L.st = take(ns * sizeof(LMSurf));
-    L.pcur = take(ns * dim * sizeof(double));
     L.ptrial = take(ns * dim * sizeof(double));
     L.jmask = take(ns * sizeof(int32_t));
     L.tmask = take(ns * sizeof(int32_t));
@@ -808,7 +826,10 @@ __global__ void k_batch_iv(const ope_contract* __restrict__ con, const double* _
 
 int launch_batch_iv(const ope_contract* con, const double* price, size_t n, double* iv, int32_t* ok, cudaStream_t st) {
     if (n == 0) return OPE_OK;
-    k_batch_iv<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(con, price, (long long)n, iv, ok);
+    // a solve is a chain of up to 70 Black-Scholes evaluations: small blocks
+    // spread a call's warps evenly (50,050 quotes per launch, 256 / 64 threads:
+    // 516 / 505 us for the whole call of 100,100)
+    k_batch_iv<<<(unsigned)((n + 63) / 64), 64, 0, st>>>(con, price, (long long)n, iv, ok);
     OPE_CHECK(cudaGetLastError());
     tctx().launches += 1;
     return OPE_OK;
@@ -824,21 +845,21 @@ int run_calib_jacobian(int model, const ope_contract* quotes, const double* iv_m
     void* ws;
     OPE_TRY(ensure_workspace(L.total, &ws, st));
     char* base = static_cast<char*>(ws);
-    std::vector<int32_t> sidx(nq);
-    for (size_t s = 0; s < ns; ++s)
-        for (int64_t i = surf_offsets[s]; i < surf_offsets[s + 1]; ++i) sidx[i] = (int32_t)s;
-    std::vector<double> wv(nq, 1.0);
-    std::vector<int32_t> ones(ns, 1);
-    OPE_CHECK(cudaMemcpyAsync(base + L.q, quotes, nq * sizeof(ope_contract), cudaMemcpyHostToDevice, st));
-    OPE_CHECK(cudaMemcpyAsync(base + L.iv, iv_market, nq * sizeof(double), cudaMemcpyHostToDevice, st));
-    OPE_CHECK(cudaMemcpyAsync(base + L.w, wv.data(), nq * sizeof(double), cudaMemcpyHostToDevice, st));
-    OPE_CHECK(cudaMemcpyAsync(base + L.off, surf_offsets, (ns + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    OPE_CHECK(cudaMemcpyAsync(base + L.sidx, sidx.data(), nq * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    OPE_CHECK(cudaMemcpyAsync(base + L.pcur, params, ns * dim * sizeof(double), cudaMemcpyHostToDevice, st));
-    OPE_CHECK(cudaMemcpyAsync(base + L.jmask, ones.data(), ns * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+    // quotes, market IVs, offsets and parameters are adjacent in the layout: one
+    // copy through the pinned buffer
+    const size_t b_in = L.w;
+    void* pin;
+    OPE_TRY(ensure_pinned(std::max(b_in, nq * (dim + 1) * sizeof(double)), &pin));
+    char* h = static_cast<char*>(pin);
+    std::memcpy(h + L.q, quotes, nq * sizeof(ope_contract));
+    std::memcpy(h + L.iv, iv_market, nq * sizeof(double));
+    std::memcpy(h + L.off, surf_offsets, (ns + 1) * sizeof(int64_t));
+    std::memcpy(h + L.pcur, params, ns * dim * sizeof(double));
+    OPE_CHECK(cudaMemcpyAsync(base, h, b_in, cudaMemcpyHostToDevice, st));
     LMDev D = make_dev(base, L, (int)nq, (int)ns, dim);
-    OPE_CHECK(cudaMemsetAsync(D.pslot, 0, ns * sizeof(int32_t), st));
-    OPE_CHECK(cudaMemsetAsync(D.jslot, 0, ns * sizeof(int32_t), st));
+    k_jac_init<<<(unsigned)((nq + ns + 255) / 256), 256, 0, st>>>(D);
+    OPE_CHECK(cudaGetLastError());
+    c.launches += 1;
     const PanelSink sink = pricing_sink(D, base, L);
     OPE_TRY(launch_price_persistent(model, D.q, nq, D.off, ns, nullptr, D.pcur, tol, D.price,
                                     carve_price_scratch(base + L.scratch, nq), st, nullptr, nullptr, &sink));
@@ -846,9 +867,12 @@ int run_calib_jacobian(int model, const ope_contract* quotes, const double* iv_m
     OPE_CHECK(cudaGetLastError());
     c.launches += 1;
     OPE_TRY(launch_jac(model, D, base, L, st));
-    OPE_CHECK(cudaMemcpyAsync(out_jac, D.jrow, nq * dim * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (out_res) OPE_CHECK(cudaMemcpyAsync(out_res, D.res, nq * sizeof(double), cudaMemcpyDeviceToHost, st));
+    const size_t b_jac = nq * dim * sizeof(double);
+    OPE_CHECK(cudaMemcpyAsync(h, D.jrow, b_jac, cudaMemcpyDeviceToHost, st));
+    if (out_res) OPE_CHECK(cudaMemcpyAsync(h + b_jac, D.res, nq * sizeof(double), cudaMemcpyDeviceToHost, st));
     OPE_CHECK(cudaStreamSynchronize(st));
+    std::memcpy(out_jac, h, b_jac);
+    if (out_res) std::memcpy(out_res, h + b_jac, nq * sizeof(double));
     return OPE_OK;
 }
 

@@ -212,6 +212,12 @@ constexpr size_t kPipelineMin = 262144;
 // pageable copy each way around the launch: a small call's time is mostly
 // these fixed costs.
 constexpr size_t kStagedMax = 16384;
+// Other small inputs and results go through the pinned buffer up to this many
+// bytes, as one copy each way.  Host memcpy + copy from pinned against a
+// pageable copy, us, host to device / back: 57 kB 12 / 13 against 46 / 18,
+// 430 kB 26 / 27 against 36 / 44, 1.1 MB 57 / 58 against 74 / 98, 2.0 MB 158 /
+// 157 against 112 / 156.
+constexpr size_t kStagedBytes = 3 << 19;
 
 // The staged small-call setup: contracts copied into the pinned buffer
 // (*k_con points at them); *h_out is the pinned slot for the prices (NULL
@@ -301,6 +307,49 @@ int price_pipelined(int model, const ope_contract* contracts, size_t n, const in
     return OPE_OK;
 }
 
+// Implied vols from pageable host memory: the second half's contracts and
+// prices copy while the first half is solved, and results of up to kStagedBytes
+// come back through the pinned buffer.  The C call on 100,100 quotes 535 ->
+// 505 us, of which the pageable copy in is some 340 (copying chunks of 16,384
+// through pinned slots instead took 642).
+int iv_pipelined(const ope_contract* contracts, size_t n, const double* prices, double* out_iv, int32_t* out_ok,
+                 ope_contract* d_con, double* d_px, double* d_iv, int32_t* d_ok) {
+    ThreadCtx& c = tctx();
+    if (!c.copy_stream) OPE_CHECK(cudaStreamCreateWithFlags(&c.copy_stream, cudaStreamNonBlocking));
+    for (auto& e : c.pipe_ev)
+        if (!e) OPE_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    cudaStream_t st = c.stream, cs = c.copy_stream;
+    // the workspace's earlier uses are ordered before st (ensure_workspace)
+    OPE_CHECK(cudaEventRecord(c.pipe_ev[0], st));
+    OPE_CHECK(cudaStreamWaitEvent(cs, c.pipe_ev[0], 0));
+    const size_t b_iv = align_up(n * sizeof(double), 256), b_out = b_iv + n * sizeof(int32_t);
+    char* h = nullptr;
+    if (b_out <= kStagedBytes) {
+        void* pin;
+        OPE_TRY(ensure_pinned(b_out, &pin));
+        h = static_cast<char*>(pin);
+    }
+    for (int part = 0; part < 2; ++part) {
+        const size_t a = part ? n / 2 : 0, cnt = (part ? n : n / 2) - a;
+        if (cnt == 0) continue;
+        OPE_CHECK(cudaMemcpyAsync(d_con + a, contracts + a, cnt * sizeof(ope_contract), cudaMemcpyHostToDevice, cs));
+        OPE_CHECK(cudaMemcpyAsync(d_px + a, prices + a, cnt * sizeof(double), cudaMemcpyHostToDevice, cs));
+        OPE_CHECK(cudaEventRecord(c.pipe_ev[1 + part], cs));
+        OPE_CHECK(cudaStreamWaitEvent(st, c.pipe_ev[1 + part], 0));
+        OPE_TRY(launch_batch_iv(d_con + a, d_px + a, cnt, d_iv + a, d_ok + a, st));
+    }
+    OPE_CHECK(cudaMemcpyAsync(h ? reinterpret_cast<double*>(h) : out_iv, d_iv, n * sizeof(double),
+                              cudaMemcpyDeviceToHost, st));
+    OPE_CHECK(cudaMemcpyAsync(h ? reinterpret_cast<int32_t*>(h + b_iv) : out_ok, d_ok, n * sizeof(int32_t),
+                              cudaMemcpyDeviceToHost, st));
+    OPE_CHECK(cudaStreamSynchronize(st));
+    if (h) {
+        std::memcpy(out_iv, h, n * sizeof(double));
+        std::memcpy(out_ok, h + b_iv, n * sizeof(int32_t));
+    }
+    return OPE_OK;
+}
+
 // Plain (one parameter set) pricing, host or device pointers.
 int batch_price(int32_t model, const ope_contract* contracts, size_t n, const void* params, double* out,
                 const ope_options* opts) {
@@ -320,6 +369,24 @@ int batch_price(int32_t model, const ope_contract* contracts, size_t n, const vo
                                        tol, out, carve_price_scratch(ws, n, b_run), user_stream(opts));
     }
     ThreadCtx& c = tctx();
+    // contracts and prices in pinned host memory are used in place (zero-copy)
+    const ope_contract* k_con = static_cast<const ope_contract*>(pinned_device_ptr(contracts));
+    double* k_out = static_cast<double*>(pinned_device_ptr(out));
+    double* h_out = nullptr;
+    if (n <= kStagedMax) {  // a small call: one launch, the parameters in its arguments
+        if (!k_con || !k_out) {
+            const ope_contract* given = k_con;
+            OPE_TRY(stage_small(contracts, n, &k_con, &k_out, &h_out));
+            if (given) k_con = given;
+        }
+        bool taken = false;
+        OPE_TRY(launch_price_row(model, k_con, n, static_cast<const double*>(params), tol, k_out, c.stream, &taken));
+        if (taken) {
+            OPE_CHECK(cudaStreamSynchronize(c.stream));
+            if (h_out) std::memcpy(out, h_out, n * sizeof(double));
+            return OPE_OK;
+        }
+    }
     const size_t b_con = align_up(n * sizeof(ope_contract), 256), b_par = 256, b_out = align_up(n * sizeof(double), 256);
     const size_t b_run = price_run_bytes(model, n, b_con + b_par + b_out + price_scratch_bytes(n));
     void* ws;
@@ -329,22 +396,10 @@ int batch_price(int32_t model, const ope_contract* contracts, size_t n, const vo
     double* d_par = reinterpret_cast<double*>(p + b_con);
     double* d_out = reinterpret_cast<double*>(p + b_con + b_par);
     void* scratch = p + b_con + b_par + b_out;
-    // contracts and prices in pinned host memory are used in place (zero-copy)
-    const ope_contract* k_con = static_cast<const ope_contract*>(pinned_device_ptr(contracts));
-    double* k_out = static_cast<double*>(pinned_device_ptr(out));
     OPE_CHECK(cudaMemcpyAsync(d_par, params, stride * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     if (!k_con && n >= kPipelineMin)
         return price_pipelined(model, contracts, n, nullptr, 1, d_par, tol, d_con, nullptr, d_out, out, k_out, nullptr,
                                nullptr, scratch, b_run);
-    double* h_out = nullptr;
-    if (!k_con && n <= kStagedMax) {
-        OPE_TRY(stage_small(contracts, n, &k_con, &k_out, &h_out));
-        OPE_TRY(launch_price_persistent(model, k_con, n, nullptr, 1, nullptr, d_par, tol, k_out,
-                                        carve_price_scratch(scratch, n, b_run), c.stream));
-        OPE_CHECK(cudaStreamSynchronize(c.stream));
-        if (h_out) std::memcpy(out, h_out, n * sizeof(double));
-        return OPE_OK;
-    }
     if (!k_con) {
         OPE_CHECK(cudaMemcpyAsync(d_con, contracts, n * sizeof(ope_contract), cudaMemcpyHostToDevice, c.stream));
         k_con = d_con;
@@ -353,6 +408,7 @@ int batch_price(int32_t model, const ope_contract* contracts, size_t n, const vo
                                     carve_price_scratch(scratch, n, b_run), c.stream));
     if (!k_out) OPE_CHECK(cudaMemcpyAsync(out, d_out, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     OPE_CHECK(cudaStreamSynchronize(c.stream));
+    if (h_out) std::memcpy(out, h_out, n * sizeof(double));
     return OPE_OK;
 }
 
@@ -388,6 +444,20 @@ int batch_greeks(int32_t model, const ope_contract* contracts, size_t n, const v
     double* d_par = reinterpret_cast<double*>(p + b_con);
     ope_pricing_result* d_out = reinterpret_cast<ope_pricing_result*>(p + b_con + b_par);
     void* gws = p + b_con + b_par + b_out;
+    if (b_con + b_par + b_out <= kStagedBytes) {  // contracts and parameters are adjacent: one copy
+        void* pin;
+        OPE_TRY(ensure_pinned(b_con + b_par + b_out, &pin));
+        char* h = static_cast<char*>(pin);
+        std::memcpy(h, contracts, n * sizeof(ope_contract));
+        std::memcpy(h + b_con, params, stride * sizeof(double));
+        OPE_CHECK(cudaMemcpyAsync(d_con, h, b_con + stride * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+        OPE_TRY(launch(d_con, d_par, d_out, gws, c.stream));
+        OPE_CHECK(cudaMemcpyAsync(h + b_con + b_par, d_out, n * sizeof(ope_pricing_result), cudaMemcpyDeviceToHost,
+                                  c.stream));
+        OPE_CHECK(cudaStreamSynchronize(c.stream));
+        std::memcpy(out, h + b_con + b_par, n * sizeof(ope_pricing_result));
+        return OPE_OK;
+    }
     OPE_CHECK(cudaMemcpyAsync(d_con, contracts, n * sizeof(ope_contract), cudaMemcpyHostToDevice, c.stream));
     OPE_CHECK(cudaMemcpyAsync(d_par, params, stride * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     OPE_TRY(launch(d_con, d_par, d_out, gws, c.stream));
@@ -522,6 +592,8 @@ int ope_batch_implied_vol(const ope_contract* contracts, size_t n, const double*
     double* d_px = reinterpret_cast<double*>(p + b_con);
     double* d_iv = reinterpret_cast<double*>(p + b_con + b_d);
     int32_t* d_ok = reinterpret_cast<int32_t*>(p + b_con + 2 * b_d);
+    if (!pinned_device_ptr(contracts))
+        return iv_pipelined(contracts, n, market_prices, out_iv, out_ok, d_con, d_px, d_iv, d_ok);
     OPE_CHECK(cudaMemcpyAsync(d_con, contracts, n * sizeof(ope_contract), cudaMemcpyHostToDevice, c.stream));
     OPE_CHECK(cudaMemcpyAsync(d_px, market_prices, n * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     OPE_TRY(launch_batch_iv(d_con, d_px, n, d_iv, d_ok, c.stream));
@@ -742,6 +814,8 @@ int ope_price_surfaces_stats(int32_t model, const ope_contract* contracts, size_
         return set_error(OPE_ERR_INVALID_ARG, "surf_offsets must start at 0 and end at n");
     for (size_t s = 0; s < n_surf; ++s)
         if (surf_offsets[s + 1] < surf_offsets[s]) return set_error(OPE_ERR_INVALID_ARG, "surf_offsets not sorted");
+    if (n_surf == 1 && n <= kStagedMax && !out_bisections)  // one surface: the plain call
+        return batch_price(model, contracts, n, params, out_prices, opts);
     ThreadCtx& c = tctx();
     const size_t b_con = align_up(n * sizeof(ope_contract), 256), b_off = align_up((n_surf + 3) * sizeof(int64_t), 256),
                  b_par = align_up(n_surf * stride * sizeof(double), 256), b_out = align_up(n * sizeof(double), 256),

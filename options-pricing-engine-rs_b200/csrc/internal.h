@@ -198,6 +198,11 @@ int launch_price_persistent(int model, const ope_contract* con, size_t n, const 
                             const PriceScratch& s, cudaStream_t st, int32_t* nbis_out = nullptr,
                             const int32_t* surf_mask = nullptr, const PanelSink* sink = nullptr,
                             const LaunchShape* shape = nullptr);
+// A small plain call of one parameter set whose row (5 or 8 doubles) is on the
+// host: one launch, the row in its arguments, no scratch.  *taken: false where
+// the current shape or size is not that kernel's (nothing launched).
+int launch_price_row(int model, const ope_contract* con, size_t n, const double* row, double tol, double* out,
+                     cudaStream_t st, bool* taken);
 // The adjoint's backward pass and combine (adjoint.cu) over panel lists a
 // pricing launch stored in `src`: out_grad (n x dim) = d price / d params.
 // bscratch: grad_backward_bytes(n, dim) bytes (chunk list, partial sums).

@@ -868,4 +868,17 @@ int launch_price_persistent(int model, const ope_contract* con, size_t n, const 
     return OPE_OK;
 }
 
+int launch_price_row(int model, const ope_contract* con, size_t n, const double* row, double tol, double* out,
+                     cudaStream_t st, bool* taken) {
+    const LaunchShape sh = price_shape(model, n);
+    *taken = n > 0 && is_small(n, false) && (sh.per_unit == 0 || sh.per_unit == 1) && sh.warps == 4 &&
+             !sh.deepest_first && sh.occupancy == 1.0 && tctx().grid_fraction == 1.0;
+    if (!*taken) return OPE_OK;
+    tctx().last_per_unit = 1;
+    tctx().last_probe = nullptr;
+    const PanelSink none{nullptr, nullptr, nullptr, 1};
+    return (model == OPE_MODEL_BATES ? launch_small<true, false> : launch_small<false, false>)(
+        con, n, nullptr, 1, nullptr, nullptr, row, tol, out, nullptr, st, nullptr, none, nullptr);
+}
+
 }  // namespace ope
