@@ -57,3 +57,24 @@ def test_nodes_beyond_the_fast_functions_range(ope, oracle):
     ref0, _ = oracle.trace_integral(con, par[:5], False, 1, 1e-10)
     got, _ = ope.trace_integral(ope.MODEL_HESTON, big, par[:5], 1, tol=1e-10)
     assert np.all(np.isfinite(got[0])) and np.max(np.abs(got[0, 9:39])) <= 1e3 * np.max(np.abs(ref0[0, 9:39]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("multiple", [1, 2, 3])
+def test_nodes_far_below_the_jump_factors_underflow(ope, oracle, multiple):
+    """A jump width that puts one node's jump exponent where 64/ln2 times it is a
+    multiple of 2^32 away from a number the exponential does not flush: the
+    factor is 0 there all the same (P2).  mu_j takes the mean jump to -1 exactly.
+    Where the factor is not 0, u mu_j is up to 1.2e5: 1.3e-11 per rounding."""
+    con = W.c1().contracts[37:38]
+    ref0, _ = oracle.trace_integral(con, np.array((0.04, 1.5, 0.04, 0.5, -0.7)), False, 1, 1e-10)
+    x = 0.5 + 0.5 * np.array([-0.9491079123427585, -0.7415311855993945, 0.0, 0.5860872354676911])
+    for t in x:  # nodes of the first panel, [0, 1]
+        u = (1.0 - t) / t
+        half = (multiple * 2.0 ** 32 - 300.0) / 92.33248261689366 / u ** 2  # sigma_j^2 / 2
+        par = np.array((0.04, 1.5, 0.04, 0.5, -0.7, 0.8, -1.5 * half, np.sqrt(2.0 * half)))
+        got, _ = ope.trace_integral(ope.MODEL_BATES, con, par, 1, tol=1e-10)
+        ref, _ = oracle.trace_integral(con, par, True, 1, 1e-10)
+        a, b = got[0, 9:39], ref[0, 9:39]
+        assert np.array_equal(np.isfinite(a), np.isfinite(b))
+        assert np.max(np.abs(a - b)) <= 1e-10 * np.max(np.abs(ref0[0, 9:39]))
