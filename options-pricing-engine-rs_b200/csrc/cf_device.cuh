@@ -25,7 +25,7 @@
 // Of Z only the phase u x depends on the strike (x = ln(S/K)); the rest is a
 // function of the node, the expiry, the rate, the parameters and the
 // integral.  So the evaluation is split: node_cf gives the strike-free part
-// (e^{Re Z} and Im Z without u x), node_finish adds one strike's phase and
+// (W and Im Z without u x), node_finish adds one strike's phase and
 // forms the value.  Contracts of one surface that share
 // an expiry and a rate share node_cf's values at every panel they both
 // bisect (the run cache of quadrature.cuh).
@@ -342,7 +342,7 @@ constexpr double kRound = 6755399441055744.0;
 // The arguments exp_node, cis_node and sin_node take must lie below 2^44 in
 // magnitude (node_range: the high word without its sign; kRangeEnd: 2^44).
 // Beyond, where a phase's own ulp passes 2^-9, and for non-finite arguments,
-// the node takes node_slow.
+// a node takes CUDA's functions (node_slow, sin_slow; the adjoint's own).
 constexpr unsigned kRangeEnd = 2u * 0x42B00000u;
 __device__ __forceinline__ unsigned node_range(double x) { return 2u * (unsigned)__double2hiint(x); }
 
@@ -576,8 +576,10 @@ __device__ __forceinline__ void csqrt_node(double zr, double zi, double& dre, do
 //   Re Z = Re C + Re D + r T + Re(-Log CF(-i)) for P1, Re C + Re D for P2
 //   Im Z = Im C + Im D + rtl u + z0im + (x u mod 2 pi)    x = ln(S/K), rtl = r T [- lambda T comp]
 //   Bates: jump = exp(jr0 - hs2 u^2 + i jmu u);  J = lt (jump - 1 - i phi comp)
-// (kept: halves of xr, -rs, zr0, zr2, zi1; ktst = 2 kts T, kts2 = 2 kts; nhv0 =
-// -sgn v0/2; z0re: every real term that is constant over the nodes)
+// (kept: halves of xr, -rs, zr0, zr2, zi1; kts2 = 2 kts; z0re: every real term
+// that is constant over the nodes; t...: with xi and d taken times T, which
+// A and, with one T in the factor tnhv0 = -sgn v0 T/2, D are free of, the
+// exponent d T and the term (xi - d) T take no product of their own)
 // The C and D of heston.rs:120-124 are formed without g = (xi - d)/(xi + d):
 // with m = (xi - d)/2, e = exp(-d T), o = 1 - e and N = d + m o (half of
 // (xi + d) - (xi - d) e),
@@ -587,13 +589,16 @@ __device__ __forceinline__ void csqrt_node(double zr, double zi, double& dre, do
 // a node takes one complex reciprocal (of N) where the literal sequence takes
 // four.
 struct CfConsts {
-    double hxr, nhrs, hzr0, hzr2, hzi1, t, kts, ktst, kts2, nhv0, rtl, z0re, z0im;
-    double jr0, hs2, jmu, lt;
+    // the fast node evaluation's: xi, z, d, m and N times T (z times T^2)
+    double thxr, tnhrs, thzr0, thzr2, thzi1, tnhv0, kts, kts2, rtl, z0re, z0im;
+    double jr0, hs2, jmu, lt, x;
     int sgn_bit;
-    // kept for the adjoint
-    double rs, sgn, phi_im, sig2, v0, rt, x, comp;
+    unsigned u_span;  // u it applies to: high words in [kULow, kULow + u_span)
+    // the same without the factor T, for the slow evaluation and the adjoint
+    double hxr, nhrs, hzr0, hzr2, hzi1, t, sgn, phi_im, v0, rt, comp;
     double z0;  // z0re without the logarithm's constant
 };
+constexpr unsigned kULow = 0x3D71979Au;  // the first high word above that of 1e-12
 
 // stable_cf at a general complex phi, following heston.rs:113-127's operation
 // order (used once per integral for the P1 normaliser CF(-i)).
@@ -628,13 +633,21 @@ __device__ __forceinline__ Cx jump_cf_ref(Cx phi, double t, double lambda, doubl
     return cexp(cscale(inner, lambda * t));
 }
 
+// Log CF(-i) by the reference's sequence; rare (make_consts), so a call.
+static __device__ __noinline__ Cx log_cf_mi_ref(double t, double r, double v0, double kappa, double theta, double sigma,
+                                                double rho, bool bates, double lambda, double mu_j, double sigma_j) {
+    const Cx phi_mi{0.0, -1.0};
+    Cx m = stable_cf_ref(phi_mi, t, r, v0, kappa, theta, sigma, rho);
+    if (bates) m = cmul(m, jump_cf_ref(phi_mi, t, lambda, mu_j, sigma_j));
+    return clog(m);
+}
+
 // Build the per-integral constants.  which: 0 = P1 (stock measure), 1 = P2.
 __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, double r, const double* p,
                                                 bool bates, int which) {
     const double v0 = p[0], kappa = p[1], theta = p[2], sigma = p[3], rho = p[4];
     CfConsts C;
-    C.rs = rho * sigma;
-    C.sig2 = sigma * sigma;
+    const double rs = rho * sigma, sig2 = sigma * sigma;
     C.kts = (kappa * theta) / (sigma * sigma);
     C.v0 = v0;
     C.t = t;
@@ -642,15 +655,22 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
     C.x = log_cr(s / k);  // heston.rs:86, rounded as the platform libm rounds it
     C.phi_im = (which == 0) ? -1.0 : 0.0;
     C.sgn = (which == 0) ? -1.0 : 1.0;
-    const double xr = kappa + C.rs * C.phi_im;
+    const double xr = kappa + rs * C.phi_im;
     C.hxr = 0.5 * xr;
-    C.nhrs = -0.5 * C.rs;
+    C.nhrs = -0.5 * rs;
     C.hzr0 = 0.5 * (xr * xr);
-    C.hzr2 = 0.5 * (C.sig2 * ((1.0 - rho) * (1.0 + rho)));
-    C.hzi1 = 0.5 * fma(-2.0 * xr, C.rs, C.sig2 * C.sgn);
+    C.hzr2 = 0.5 * (sig2 * ((1.0 - rho) * (1.0 + rho)));
+    C.hzi1 = 0.5 * fma(-2.0 * xr, rs, sig2 * C.sgn);
     C.kts2 = 2.0 * C.kts;
-    C.ktst = C.kts2 * t;
-    C.nhv0 = -0.5 * v0 * C.sgn;
+    C.tnhv0 = -0.5 * v0 * C.sgn * t;
+    // from the rounded xr T, rs T and sigma T, so that z stays the square (and xi
+    // the root) of one xi and d cancels against it as without the factor
+    const double tsg = sigma * t, ts2 = 0.5 * (tsg * tsg);
+    C.thxr = C.hxr * t;
+    C.tnhrs = C.nhrs * t;
+    C.thzr0 = 2.0 * (C.thxr * C.thxr);
+    C.thzr2 = ts2 * ((1.0 - rho) * (1.0 + rho));
+    C.thzi1 = fma(4.0 * C.thxr, C.tnhrs, ts2 * C.sgn);
     C.sgn_bit = which == 0 ? (int)0x80000000 : 0;
     double lt = 0.0, mu_j = 0.0, hs2 = 0.0, comp = 0.0;
     if (bates) {
@@ -676,16 +696,14 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
         // non-finite parameter -- it is evaluated with the reference's own
         // sequence.  (The regular case skips two complex exponentials, three
         // complex divisions and two complex logarithms per P1 integral.)
-        bool regular = xr > 1e-100 && xr < 1e100 && C.sig2 > 1e-100 && C.kts < 1e4 &&
-                       v0 / (sigma * sigma) * xr < 1e4 && fabs(C.rt) < 700.0 && t < 1e3;
+        bool regular = xr > 1e-100 && xr < 1e100 && sig2 > 1e-100 && C.kts < 1e4 &&
+                       v0 * xr < 1e4 * sig2 && fabs(C.rt) < 700.0 && t < 1e3;
         if (bates) regular = regular && fabs(p[6] + 0.5 * p[7] * p[7]) < 50.0 && fabs(lt) * (comp + 1.0) < 1e4;
         if (regular) {
             lnm_re = -C.rt;
         } else {
-            const Cx phi_mi{0.0, -1.0};
-            Cx m = stable_cf_ref(phi_mi, t, r, v0, kappa, theta, sigma, rho);
-            if (bates) m = cmul(m, jump_cf_ref(phi_mi, t, p[5], p[6], p[7]));
-            Cx lm = clog(m);
+            const Cx lm = log_cf_mi_ref(t, r, v0, kappa, theta, sigma, rho, bates, bates ? p[5] : 0.0,
+                                        bates ? p[6] : 0.0, bates ? p[7] : 0.0);
             lnm_re = -lm.re;
             lnm_im = -lm.im;
         }
@@ -693,6 +711,16 @@ __device__ __forceinline__ CfConsts make_consts(double s, double k, double t, do
     C.z0 = (-C.rt * C.phi_im + lnm_re) + lt * (C.phi_im * comp - 1.0);
     C.z0re = fma(C.kts, 0.6931471805599453, C.z0);
     C.z0im = lnm_im;
+    // Where the fast evaluation applies, as a range of u: T > 1e-9 and |rho| <= 1
+    // (Re z >= 0), a finite normaliser, u >= 1e-12, and every argument of its
+    // functions that a bound on u bounds below 2^43: |d| T <= T (|xr| + 2 r1 +
+    // r2) max(u, 1) with r1^2 = |zi1|, r2^2 = zr2 (and 2 sqrt y <= 1 + y), |jmu| u,
+    // |jr0| + hs2 u^2.
+    const float tf = (float)t, h2 = (float)C.hs2;
+    const float q = tf * (2.0f + (float)(fabs(xr) + fma(2.0, fabs(C.hzi1), C.hzr2))) + (float)(fabs(C.jmu) + fabs(C.jr0));
+    const bool fast = tf > 1e-9f && C.hzr2 >= 0.0 && q < 8.796e12f && h2 < 8.796e12f && isfinite(C.z0re) && isfinite(C.z0im);
+    const float top = fminf(__fdividef(8.79e12f, q), 2.9e6f * rsqrtf(h2));
+    C.u_span = fast && top > 1e-3f ? (unsigned)__double2hiint((double)fminf(top, 1e30f)) - kULow : 0u;
     return C;
 }
 
@@ -710,11 +738,10 @@ __device__ __forceinline__ double node_u(double omt, double tn, double itt) {
 }
 
 // The strike-free part of a node (heston.rs:221-227 with the merged-exponent
-// integrand): E = e^{Re Z}, A = Im Z - (u x mod 2 pi), and the node's
-// u = (1 - t)/t and itt = 1/((1 - t) t) (node_geom computes the last two
-// alone, bit for bit).
+// integrand): W = e^{Re Z} / ((1 - t) t), A = Im Z - (u x mod 2 pi), and the
+// node's u = (1 - t)/t (which node_geom computes alone, bit for bit).
 struct NodeCf {
-    double e, a, u, itt;
+    double w, a, u;
 };
 
 __device__ __forceinline__ void node_geom(double tn, double& u, double& itt) {
@@ -730,10 +757,10 @@ __device__ __forceinline__ double node_u_of(double tn) {
     return u;
 }
 
-// FAST: branch-free, with the functions above; `range` receives what decides
-// whether they applied (compare with kRangeEnd): the largest of their
-// arguments, and the sign of Re z (negative only for |rho| > 1).  Not FAST:
-// CUDA's functions and the square root's other branch.
+// FAST: branch-free, with the functions above; returns whether they applied: u
+// in the integral's range (CfConsts::u_span) and Z below 2^43, its real part
+// below 700 (so that the value is finite).  Not FAST: CUDA's functions and the
+// square root's other branch.
 //
 // What bounds it: register-file reads and issue slots (an FMA of three
 // different registers takes 3 cycles of a scheduler's operand reads, of two
@@ -748,16 +775,21 @@ __device__ __forceinline__ double node_u_of(double tn) {
 //    9.66 /  8.45  21-bit leading coefficients and reductions
 //    9.36 /  7.88  N and o as below, arg_node's rotation, integer clamps in
 //                  exp_node (Heston at 72 registers; 8.12 at 64)
+//    9.05 /  7.61  (the step's argmax)
+//    8.45 /  7.43  everything times T, one test of u for the arguments, no
+//                  tests on the value, the normaliser's general form a call
+//                  (both at 72 registers)
 // Two integrals per warp side by side (128 registers) issue 13 % fewer
 // instructions and read as many registers: 9.61 / 8.60 ms against 9.74 / 8.60.
 template <bool BATES, bool FAST>
-__device__ __forceinline__ NodeCf node_eval(const CfConsts& C, double tn, unsigned& range) {
+__device__ __forceinline__ bool node_eval(const CfConsts& C, double tn, NodeCf& n) {
     double u, itt;  // (1 - t) / t and 1 / ((1 - t) t)
     node_geom(tn, u, itt);
     const double u2 = __dmul_rn(u, u);
     // xi/2 = (hxr, hxi); z/2, z = xi^2 + sigma^2 phi(phi+i) = (xr^2 + zr2 u^2, zi1 u)
-    const double hxi = __dmul_rn(C.nhrs, u);
-    const double zr = fma(C.hzr2, u2, C.hzr0), zi = __dmul_rn(C.hzi1, u);
+    const double hxr = FAST ? C.thxr : C.hxr, hxi = __dmul_rn(FAST ? C.tnhrs : C.nhrs, u);
+    const double zr = FAST ? fma(C.thzr2, u2, C.thzr0) : fma(C.hzr2, u2, C.hzr0);
+    const double zi = __dmul_rn(FAST ? C.thzi1 : C.hzi1, u);
     // d = sqrt z: Re d = sqrt(|z/2| + Re z/2), Im d = (Im z/2) / Re d
     const double zz = fma(zr, zr, __dmul_rn(zi, zi));
     const double az = __dmul_rn(zz, rsqrt_nr(zz));  // |z| / 2
@@ -769,18 +801,17 @@ __device__ __forceinline__ NodeCf node_eval(const CfConsts& C, double tn, unsign
         dre = fabs(dim);
         dim = copysign(w, zi);
     }
-    const double mr = fma(dre, -0.5, C.hxr), mi = fma(dim, -0.5, hxi);  // m = (xi - d) / 2
-    // e = exp(-d T), o = 1 - e
-    const double th = __dmul_rn(-dim, C.t), et = __dmul_rn(-dre, C.t);
+    const double mr = fma(dre, -0.5, hxr), mi = fma(dim, -0.5, hxi);  // m = (xi - d) / 2
+    // e = exp(-d T) = em (ec - i es), o = 1 - e
     double em, ec, es;
     if (FAST) {
-        cis_node(th, ec, es);
-        em = exp_node(et);
+        cis_node(dim, ec, es);
+        em = exp_node(-dre);
     } else {
-        sincos(th, &es, &ec);
-        em = exp(et);
+        sincos(dim * C.t, &es, &ec);
+        em = exp(-dre * C.t);
     }
-    const double omr = fma(-em, ec, 1.0), omi = __dmul_rn(-em, es);
+    const double omr = fma(-em, ec, 1.0), omi = __dmul_rn(em, es);
     // N = d + m o
     const double nr = fma(-mi, omi, fma(mr, omr, dre));
     const double ni = fma(mr, omi, fma(mi, omr, dim));
@@ -792,16 +823,15 @@ __device__ __forceinline__ NodeCf node_eval(const CfConsts& C, double tn, unsign
     // D = -(v0/2) phi(phi+i) o / N, phi(phi+i) = u (u + i sgn) = sgn u (sgn u + i)
     const double qr = fma(omr, nr, __dmul_rn(omi, ni)), qi = fma(omi, nr, __dmul_rn(-omr, ni));
     const double su = __hiloint2double(__double2hiint(u) | C.sgn_bit, __double2loint(u));
-    const double s = __dmul_rn(__dmul_rn(C.nhv0, u), ia);
+    const double s = __dmul_rn(__dmul_rn(FAST ? C.tnhv0 : -0.5 * C.v0 * C.sgn, u), ia);
     // Re, Im Z = kts ((xi - d) T - 2 Log A) + D + z0 + i (r T u)
-    double zre = fma(C.ktst, mr, fma(-C.kts, la, fma(s, fma(su, qr, -qi), C.z0re)));
-    double zim = fma(C.ktst, mi, fma(-C.kts2, li, fma(s, fma(su, qi, qr), fma(C.rtl, u, C.z0im))));
-    if (FAST) range = max(node_range(et), (unsigned)__double2hiint(zr));  // Re z < 0: above kRangeEnd
+    const double km = FAST ? C.kts2 : C.kts2 * C.t;
+    double zre = fma(km, mr, fma(-C.kts, la, fma(s, fma(su, qr, -qi), C.z0re)));
+    double zim = fma(km, mi, fma(-C.kts2, li, fma(s, fma(su, qi, qr), fma(C.rtl, u, C.z0im))));
     if (BATES) {
         const double tj = __dmul_rn(C.jmu, u), ej = fma(-C.hs2, u2, C.jr0);
         double jc, js, je;
         if (FAST) {
-            range = max(range, max(node_range(tj), node_range(ej)));
             cis_node(tj, jc, js);
             je = __dmul_rn(C.lt, exp_node(ej));
         } else {
@@ -811,23 +841,32 @@ __device__ __forceinline__ NodeCf node_eval(const CfConsts& C, double tn, unsign
         zre = fma(je, jc, zre);
         zim = fma(je, js, zim);
     }
-    if (FAST) range = max(range, node_range(zre));
-    return NodeCf{FAST ? exp_node(zre) : exp(zre), zim, u, itt};
+    n.u = u;
+    n.a = zim;
+    n.w = __dmul_rn(FAST ? exp_node(zre) : exp(zre), itt);
+    if (!FAST) return true;
+    const int hz = __double2hiint(zre);
+    return (unsigned)__double2hiint(u) - kULow < C.u_span && hz < 0x4085E000 && (unsigned)hz < 0xC2A00000u &&
+           node_range(zim) < 2u * 0x42A00000u;
 }
 
-// The rare nodes out of the fast functions' range (internal linkage: within
-// the calling kernel's register budget).
+// The rare nodes the fast evaluation does not apply to (internal linkage:
+// within the calling kernel's register budget): W = 0 where the reference's g(t)
+// is 0 (t <= 0, u < 1e-12) or W or the phase is not finite, and a phase beyond
+// 2^44, whose last place passes 2^-9, brought below 2 pi.
 template <bool BATES>
 static __device__ __noinline__ NodeCf node_slow(const CfConsts& C, double tn) {
-    unsigned range;
-    return node_eval<BATES, false>(C, tn, range);
+    NodeCf n;
+    node_eval<BATES, false>(C, tn, n);
+    if (!(tn > 0.0 && n.u >= 1e-12 && isfinite(n.w) && isfinite(n.a))) return NodeCf{0.0, 0.0, 0.0};
+    if (fabs(n.a) >= 0x1p44) n.a = fmod(n.a, 6.283185307179586);
+    return n;
 }
 
 template <bool BATES>
 __device__ __forceinline__ NodeCf node_cf(const CfConsts& C, double tn) {
-    unsigned range;
-    NodeCf n = node_eval<BATES, true>(C, tn, range);
-    if (range >= kRangeEnd) n = node_slow<BATES>(C, tn);
+    NodeCf n;
+    if (!node_eval<BATES, true>(C, tn, n)) n = node_slow<BATES>(C, tn);
     return n;
 }
 
@@ -842,35 +881,19 @@ __device__ __forceinline__ NodeCf node_cf(const CfConsts& C, double tn) {
 // u x is.  The reference adds the two phases exactly too, through the
 // complex product e^{iux} CF (an unreduced sum would lose ulp(u x), 1e-9 at
 // u x = 1e7, on short-dated deep-wing contracts).
-// LIVE_IN_W: w already carries the liveness (NaN where the node is not live,
-// see node_w_live), as the run cache stores it; the value is then 0 exactly
-// where the explicit test gives 0.
+// W is 0 where that value is to be 0 (node_slow), so only a phase u x that is
+// out of sin_node's range or not finite needs a test.
 static __device__ __noinline__ double sin_slow(double ux, double a, double w) {
     const double nq = rint(ux * 0.15915494309189535);  // 1 / (2 pi)
     const double uxr = fma(-nq, 2.4492935982947064e-16, fma(-nq, 6.283185307179586, ux));
-    return __dmul_rn(sin(__dadd_rn(a, uxr)), w);
+    const double v = __dmul_rn(sin(__dadd_rn(a, uxr)), w);
+    return isfinite(v) ? v : 0.0;
 }
-template <bool LIVE_IN_W = false>
-__device__ __forceinline__ double node_finish_w(double x, double tn, double w, double a, double u) {
+__device__ __forceinline__ double node_finish(double x, double u, double a, double w) {
     const double ux = __dmul_rn(u, x);
     double v = sin_node(ux, a, w);
-    if (max(node_range(ux), node_range(a)) >= kRangeEnd) v = sin_slow(ux, a, w);
-    const bool ok = (LIVE_IN_W || u >= 1e-12) && isfinite(v);
-    return ok ? v : 0.0;
+    if (node_range(ux) >= kRangeEnd) v = sin_slow(ux, a, w);
+    return v;
 }
-
-// W with the node's liveness folded in: NaN where the reference's g(t) is 0
-// whatever the strike (t <= 0, u < 1e-12).
-__device__ __forceinline__ double node_w_live(double tn, const NodeCf& n) {
-    return ((tn > 0.0) && (n.u >= 1e-12)) ? __dmul_rn(n.e, n.itt) : __longlong_as_double(0x7ff8000000000000ll);
-}
-
-__device__ __forceinline__ double node_w(const NodeCf& n) { return __dmul_rn(n.e, n.itt); }
-
-__device__ __forceinline__ double node_finish(double x, double tn, const NodeCf& n) {
-    return node_finish_w(x, tn, node_w(n), n.a, n.u);
-}
-
-
 
 }  // namespace ope

@@ -24,18 +24,18 @@
 // Register budget of the pricing kernel: per model, the minimum resident
 // blocks per SM of the 4-warp shape handed to __launch_bounds__ (registers
 // per thread capped at 65536 / (32 * 4 * MINB)); the 1- and 2-warp shapes get
-// 4 / warps times as many blocks.  262k wing contracts, 8 / 7 blocks (64 / 72
-// registers): Bates 9.36 / 9.40 ms, Heston 8.12 / 7.88 ms.
+// 4 / warps times as many blocks.  262k wing contracts at 8 / 7 / 6 blocks (64
+// to 80 registers), ms: Bates 8.71 / 8.45 / 8.62, Heston 7.41 / 7.43 / 7.56.
 #ifndef OPE_KERNEL_MINB_BATES
-#define OPE_KERNEL_MINB_BATES 8
+#define OPE_KERNEL_MINB_BATES 7
 #endif
 #ifndef OPE_KERNEL_MINB_HESTON
 #define OPE_KERNEL_MINB_HESTON 7
 #endif
-// The same for the run kernel (both models): 8 / 7 blocks 27.1 / 32.8 ms on
-// 1.46M grid contracts.
+// The same for the run kernel (both models): 7 / 6 / 5 blocks 22.5 / 22.0 / 22.5
+// ms on 1.46M grid contracts.
 #ifndef OPE_RUNS_MINB
-#define OPE_RUNS_MINB 8
+#define OPE_RUNS_MINB 6
 #endif
 
 namespace ope {
@@ -160,25 +160,42 @@ __device__ __forceinline__ ContractView load_contract(const ope_contract* con, l
     return v;
 }
 
+// A unit's integrand constants into the warp's shared copy.  In line: as a call,
+// 262k Bates wings took 8.56 ms instead of 8.45, Heston 7.50 instead of 7.43, and
+// the pricing of 19,200 calibration quotes (ten short integrals a warp) 196 us
+// instead of 187; the run kernel 21.4 ms instead of 22.0.
+template <bool BATES>
+__device__ __forceinline__ void load_unit(long long c, int which, const ope_contract* con, const double* p, CfConsts& Cs,
+                                       int lane) {
+    const ContractView v = load_contract(con, c, lane);
+    double pl[8];
+#pragma unroll
+    for (int i = 0; i < (BATES ? 8 : 5); ++i) pl[i] = __ldg(p + i);
+    const CfConsts Cl = make_consts(v.s, v.k, v.t, v.r, pl, BATES, which);
+    __syncwarp();
+    if (lane == 0) Cs = Cl;
+    __syncwarp();
+}
+
 // Integrate unit (contract c, integral `which`) and, if it completes the
 // contract, write the price.  SAVE: also store the final live-panel list
 // and the bisection count in `sink` (slot `slot`), for the adjoint's backward
 // pass.
-// CACHED: through the run cache `rc` (the run kernel).
+// CACHED: through the run cache `rc` (the run kernel); `same`: Cs holds the
+// constants of a contract of the same run, of which only x = ln(S/K) changes.
 template <bool BATES, bool SAVE, bool CACHED = false>
 __device__ __forceinline__ void run_unit(long long c, int which, const ope_contract* con, const double* p,
                                          double tol, double* out, double* integ, unsigned int* done,
                                          int32_t* nbis_out, const PanelSink& sink, int slot, PanelStore& L,
-                                         CfConsts& Cs, int lane, const LaneRule& R, RunCacheWarp* rc = nullptr) {
-    {
-        const ContractView v = load_contract(con, c, lane);
-        double pl[8];
-#pragma unroll
-        for (int i = 0; i < (BATES ? 8 : 5); ++i) pl[i] = __ldg(p + i);
-        const CfConsts Cl = make_consts(v.s, v.k, v.t, v.r, pl, BATES, which);
+                                         CfConsts& Cs, int lane, const LaneRule& R, RunCacheWarp* rc = nullptr,
+                                         bool same = false) {
+    if (CACHED && same) {
+        const double x = log_cr(__ldg(&con[c].spot) / __ldg(&con[c].strike));
         __syncwarp();
-        if (lane == 0) Cs = Cl;
+        if (lane == 0) Cs.x = x;
         __syncwarp();
+    } else {
+        load_unit<BATES>(c, which, con, p, Cs, lane);
     }
     const CfConsts& C = Cs;
     int nb;
@@ -355,11 +372,11 @@ __global__ void __launch_bounds__(64, 8)
 // Prices are bit-identical to k_price_persistent's.
 //
 // What bounds it: issue slots (77 % used), most of them the step's bookkeeping
-// (344 instructions per step, of which 85 FP64).  Without a per-run switch, with
+// (350 instructions per step, of which 100 FP64).  Without a per-run switch, with
 // a node's (W, A) as one 16-byte word, a sentinel entry in place of branches and
 // the node evaluation inline again (out of line, a miss saved and restored the
 // loop's registers through local memory): 24.7 -> 23.3 ms on 1.46M Heston grid
-// contracts (23.9 ms out of line; inline at 7 / 6 blocks 28.9 / 23.9 ms).
+// contracts; ln(S/K) alone anew for a run's later strikes, 80 registers: 22.0 ms.
 struct RunCacheMem {
     double2* vals;  // per warp of the grid: [cap][16] (w, a)
     int cap;
@@ -423,7 +440,7 @@ __global__ void __launch_bounds__(WARPS * 32, OPE_RUNS_MINB * 4 / WARPS)
             }
             if (!param_idx && n_surf > 1 && !ope_check(s >= 0 && s < n_surf, CHK_SURFACE)) continue;
             run_unit<BATES, false, true>(c, which, con, params + s * stride, tol, out, integ, done, nbis_out, none,
-                                         0, smem_panels[warp], s_consts[warp], lane, R, &rc);
+                                         0, smem_panels[warp], s_consts[warp], lane, R, &rc, !((starts >> i) & 1u));
         }
     }
 }

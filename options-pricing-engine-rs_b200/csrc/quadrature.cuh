@@ -125,7 +125,7 @@ __device__ __forceinline__ double gk_sums(double f, const LaneRule& R) {
 // its entry (kNoEntry: not cached, nor are its descendants), so a bisection
 // finds its children's values with one load, without searching.  A contract
 // whose next panel is in the tree skips node_cf (the CF, its square root,
-// logarithm and exponentials) and pays only node_finish_w (its own phase and
+// logarithm and exponentials) and pays only node_finish (its own phase and
 // one sine).  The tree lives in global memory (per warp: cap entries of 15
 // nodes x {W, A}); when it is full, further panels are evaluated
 // uncached.  The cached values are the ones node_cf's result gives (u is
@@ -138,7 +138,7 @@ constexpr int kNoEntry = 127;       // not cached; as an entry it has no childre
 constexpr int kRunLinks = 128;
 
 struct RunCacheWarp {
-    double2* wa;     // [cap][16]: W = e^{Re Z} / ((1 - t) t), NaN at nodes that are not live, and Im Z without the phase
+    double2* wa;     // [cap][16]: W and Im Z without the phase (NodeCf)
     uint8_t* child;  // shared, [kRunLinks]: left child's entry, the right one's is the next (kNoEntry: none yet)
     uint8_t* slot;   // shared, [kMaxPanels]: entry of each live panel of the running integral
     int cap;         // entries (1..kRunEntries)
@@ -249,14 +249,14 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
             nu = node_u_of(tn);
         } else {
             const NodeCf nc = node_cf<BATES>(C, tn);
-            nw = CACHED ? node_w_live(tn, nc) : node_w(nc);
+            nw = nc.w;
             na = nc.a;
             nu = nc.u;
             // each half-warp writes its child's entry whole, pad lane included
             if (CACHED && put && (len > 0 || R.half == 0))
                 __stcg(rc->wa + (el_ + R.half) * 16 + (lane & 15), make_double2(nw, na));
         }
-        const double f = node_finish_w<CACHED>(C.x, tn, nw, na, nu);
+        const double f = node_finish(C.x, nu, na, nw);
         // K (in the lanes with bit 3 clear) and error of this half's child,
         // then both children's sums
         const double v = gk_sums(f, R);
