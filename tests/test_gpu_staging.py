@@ -59,9 +59,9 @@ def test_greeks_on_both_sides_of_the_staging_limit(ope, analytic):
     assert np.array_equal(a, b[:13100])
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 4097, 131073])
+@pytest.mark.parametrize("n", [1, 2, 3, 4097, 16385, 131073])
 def test_implied_vols_in_two_parts(ope, oracle, n):
-    """131,073 is past what the results' pinned buffer takes.  The solver stops
+    """Up to 4,097 go in one part; 131,073 is past what the results' pinned buffer takes.  The solver stops
     within 1e-10 of the price; these quotes' vegas are S sqrt(T) phi(d1) >= 3
     (T >= 0.1, |d1| <= 1.5), so the vols lie within 1e-10 / 3 of the true ones;
     the bar is 1e-9."""
