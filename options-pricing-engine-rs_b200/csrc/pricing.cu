@@ -50,7 +50,7 @@ constexpr size_t kHistBytes = (2 * kOrderBuckets + kSmSlots) * sizeof(unsigned i
 #define OPE_RUN_CACHE_ENTRIES kRunEntries
 #endif
 constexpr int kRunCacheEntries = OPE_RUN_CACHE_ENTRIES;
-constexpr int kRunWarpsPerSm = 32;
+constexpr int kRunWarpsPerSm = 4 * OPE_RUNS_MINB;
 // Automatic launches (per_unit 0): calls large enough for kRunsMinPerUnit
 // contracts per unit (worth_probing) probe for runs (k_run_probe), which picks
 // kRunsMinPerUnit to kRunsMaxPerUnit contracts per unit, or the per-contract
@@ -58,17 +58,21 @@ constexpr int kRunWarpsPerSm = 32;
 constexpr int kRunsMinPerUnit = 4;
 constexpr int kRunsMaxPerUnit = 16;
 // Units every warp of the run kernel's grid is to have at `pu` contracts per
-// unit, so that the tail of a queue of long units stays short.  1 / 4 / 8 / 16
-// contracts per unit on Heston grids, ms: 92,529 contracts 1.98 / 2.04 / 2.27 /
-// 2.88, 177,518 3.83 / 3.68 / 4.34 / 6.01, 373,066 8.13 / 6.87 / 7.31 / 8.58,
-// 510,832 11.02 / 9.06 / 9.05 / 10.00, 1,459,714 31.6 / 24.9 / 23.1 / 22.9.
-__host__ __device__ constexpr int runs_units_per_warp(int pu) { return pu < 8 ? 16 : 28; }
+// unit, so that the tail of a queue of long units stays short.  1 (deepest-first
+// below 355,200) / 4 / 8 / 16 contracts per unit on Heston grids, ms: 45,689
+// contracts 0.97 / 1.33 / 1.82 / 2.77, 92,529 1.94 / 1.89 / 2.11 / 2.66, 177,518
+// 3.74 / 3.35 / 3.97 / 5.54, 373,066 7.95 / 6.61 / 6.71 / 7.68, 510,832 10.8 / 8.73 /
+// 8.57 / 9.25, 724,573 15.3 / 12.5 / 12.0 / 12.5, 1,459,714 30.9 / 24.2 / 22.1 / 21.9;
+// Bates 92,529 2.25 / 2.03 / 2.29 / 2.91, 373,066 9.04 / 6.88 / 6.91 / 7.90.
+// 28 for 8 and 16 rather than 32 and 40: 447,420 Heston 7.60 against 7.73, Bates
+// 7.83 against 8.14, 1,066,555 Bates 16.7 against 17.1.
+__host__ __device__ constexpr int runs_units_per_warp(int pu) { return pu < 8 ? 12 : 28; }
 constexpr size_t kRunCacheWarpBytes = (size_t)kRunCacheEntries * 2 * 16 * sizeof(double);
 constexpr size_t kRunSharedBytes = (kMaxPanels + kRunLinks + 15) / 16 * 16;  // per warp: slots, child links
 
 // Whether the run probe could choose the run kernel: blocks of
 // kRunsMinPerUnit contracts must leave every warp of its grid its units
-// (151,552 contracts on 148 SMs).
+// (85,248 contracts on 148 SMs).
 bool worth_probing(size_t n) {
     int sms = 0;
     if (current_device_sms(&sms) != OPE_OK) return false;

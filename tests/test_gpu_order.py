@@ -62,3 +62,25 @@ def test_automatic_order_prices_as_input_order(ope, model, contracts_per_sm):
         ope.set_autotune(True)
     assert np.array_equal(auto, _in_input_order(ope, m, w))
     assert np.array_equal(graded, auto)
+
+
+@pytest.mark.parametrize("short", [1, 0])
+@pytest.mark.parametrize("model", ["heston", "bates"])
+def test_smallest_call_that_shares_runs(ope, model, short):
+    """Runs of 32 equal expiries are shared from 576 contracts per SM: the same
+    prices on both sides, bit for bit."""
+    m = ope.MODEL_BATES if model == "bates" else ope.MODEL_HESTON
+    n = 576 * ope.device_info()[0] - short
+    w = W.c3(n=n, per_surface=4096, seed=3)
+    if model == "heston":
+        w.params = np.ascontiguousarray(w.params[:, :5])
+    for f in ("expiry", "rate"):
+        w.contracts[f] = w.contracts[f][np.arange(n) // 32 * 32]
+    ope.set_autotune(False)
+    try:
+        got = ope.price_surfaces(m, w.contracts, w.surf_offsets, w.params, tol=w.tol)
+        used = ope.last_per_unit()
+    finally:
+        ope.set_autotune(True)
+    assert used == (1 if short else 4)
+    assert np.array_equal(got, _in_input_order(ope, m, w))
