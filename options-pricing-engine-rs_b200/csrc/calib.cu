@@ -539,8 +539,8 @@ Layout layout(size_t nq, size_t ns, int dim) {
     L.res = take(nq * sizeof(double));
     L.res_new = take(nq * sizeof(double));
     L.jrow = take(nq * dim * sizeof(double));
-    L.iv_cur = take(nq * sizeof(double));
-    L.iv_new = take(nq * sizeof(double));
+    L.iv_cur = take(2 * nq * sizeof(double));
+    L.iv_new = L.iv_cur + nq * sizeof(double);
     L.counters = take(4 * sizeof(unsigned int));
     L.out = take(ns * sizeof(ope_calib_result));
     L.prior = take(ns * dim * sizeof(double));

@@ -117,8 +117,8 @@ struct PriceScratch {
     unsigned int* done;            // n   (must be zero before launch)
     unsigned long long* head;      // 1   (must be zero before launch; persistent only)
     uint32_t* order = nullptr;     // n   queue position -> contract
-    uint32_t* bucket = nullptr;    // n   depth bucket of each contract
-    unsigned int* hist = nullptr;  // 2 x 64 bucket counts and fill counters, resident-block counters
+    uint32_t* bucket = nullptr;    // n   depth bucket of each contract, then resident-block counters
+    unsigned int* hist = nullptr;  // 2 x 64 bucket counts and fill counters
     // run cache of the run kernel (optional; run_cache_bytes() bytes): without
     // it a launch takes one contract per unit whatever its shape asks
     void* runcache = nullptr;

@@ -42,8 +42,8 @@ namespace ope {
 
 namespace {
 constexpr int kOrderBuckets = 64;
-constexpr int kSmSlots = 256;  // resident-block counters, by %smid
-constexpr size_t kHistBytes = (2 * kOrderBuckets + kSmSlots) * sizeof(unsigned int);
+constexpr int kSmSlots = 256;  // resident-block counters, by %smid (in the order's bucket array)
+constexpr size_t kHistBytes = 2 * kOrderBuckets * sizeof(unsigned int);
 // Run cache entries per warp (panels of one run), and warps per SM it is
 // sized for (the 64-register budget holds at most 32).
 #ifndef OPE_RUN_CACHE_ENTRIES
@@ -81,7 +81,7 @@ bool worth_probing(size_t n) {
 }
 
 // Layout: integ (2n doubles) | done (n) | head (256 B) | hist (2 x kOrderBuckets
-// counters, then kSmSlots resident-block counters) | order (n) | bucket (n);
+// counters) | order (n) | bucket (n);
 // done, head and hist are adjacent so one memset clears them.
 size_t price_scratch_bytes(size_t n) {
     return align_up(2 * n * sizeof(double), 256) + align_up(n * sizeof(unsigned int), 256) + 256 + kHistBytes +
@@ -577,7 +577,8 @@ __device__ __forceinline__ float depth_estimate(int b) {
 // exclusive prefix sum of the kOrderBuckets counts hist[0..64), one warp),
 // then each contract takes the next free slot of its bucket through the fill
 // counters hist[64..128) (the order inside a bucket is arbitrary, and
-// irrelevant to the prices).
+// irrelevant to the prices).  The buckets, once read, are zeroed: the pricing
+// kernel counts its resident blocks there.
 //
 // sms > 0: block 0 also leaves in head[1] how many warps of the pricing kernel
 // are to stay resident on each SM (0: all, negative: that many fewer).  A chain's step takes the longer the more warps
@@ -591,7 +592,7 @@ __device__ __forceinline__ float depth_estimate(int b) {
 // (29), 32,768 1.141 / 1.221 (57), 65,536 2.270 / 2.270 (114); Heston grids of
 // 22,654 contracts 0.524 / 0.551.  Input order and all blocks: 0.398, 0.506,
 // 0.822, 1.294, 2.435; 0.594.
-__global__ void __launch_bounds__(256) k_order_scatter(long long n, const uint32_t* __restrict__ bucket,
+__global__ void __launch_bounds__(256) k_order_scatter(long long n, uint32_t* __restrict__ bucket,
                                                        unsigned int* hist, uint32_t* __restrict__ order,
                                                        unsigned long long* head, int sms) {
     __shared__ unsigned int start[kOrderBuckets];
@@ -624,6 +625,7 @@ __global__ void __launch_bounds__(256) k_order_scatter(long long n, const uint32
     unsigned int* fill = hist + kOrderBuckets;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
         const uint32_t b = bucket[c];
+        bucket[c] = 0;
         order[start[b] + atomicAdd(fill + b, 1u)] = (uint32_t)c;
     }
 }
@@ -638,7 +640,7 @@ constexpr size_t kOrderMinPerSm = 16, kOrderMaxPerSm = 2400;
 bool order_by_size(size_t n, size_t n_surf, const int32_t* param_idx) {
     int sms = 0;
     if (n_surf <= 1 || param_idx || current_device_sms(&sms) != OPE_OK) return false;
-    return n >= kOrderMinPerSm * sms && n < kOrderMaxPerSm * sms;
+    return n >= std::max<size_t>(kOrderMinPerSm * sms, kSmSlots) && n < kOrderMaxPerSm * sms;
 }
 
 // Calls k_price_small takes instead of the persistent grid: up to 48 contracts
@@ -680,7 +682,7 @@ int launch_impl(const ope_contract* con, size_t n, const int64_t* surf_offsets, 
     OPE_TRY(current_device_sms(&sms));
     k_price_persistent<BATES, SAVE, WARPS><<<grid, threads, smem, st>>>(
         con, (long long)n, surf_offsets, (long long)n_surf, param_idx, surf_mask, params, tol, out, s.integ, s.done,
-        s.head, nbis_out, sink, order, s.hist + 2 * kOrderBuckets, grid / sms);
+        s.head, nbis_out, sink, order, s.bucket, grid / sms);
     OPE_CHECK(cudaGetLastError());
     return OPE_OK;
 }
