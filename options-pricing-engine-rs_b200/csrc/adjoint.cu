@@ -171,7 +171,9 @@ __global__ void __launch_bounds__(128, BATES ? OPE_GRAD_MINB_BATES : OPE_GRAD_MI
         const double* P = src.panels + pidx * (2 * kMaxPanels) + 2 * p0;
         double acc[DIM];
         const int items = 15 * max(p1 - p0, 0);
-        for (bool fast = true;; fast = false) {
+        // a coefficient of the chain that is not finite (sigma = 0, say) makes
+        // every node's derivatives so: the sums alone would not show it
+        for (bool fast = isfinite(G.tis2 + G.kis2 + G.sk);; fast = false) {
             double sum[DIM];
 #pragma unroll
             for (int k = 0; k < DIM; ++k) sum[k] = 0.0;
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(128, BATES ? OPE_GRAD_MINB_BATES : OPE_GRAD_MI
                     const double tn = __dadd_rn(cc, __dmul_rn(h, xj));
                     if (!(fast && node_sums<BATES, true>(C, G, tn, h * wj, sum))) {
                         double g[DIM];
-                        node_sums_slow<BATES>(C, G, tn, h * wj, g);
+                        node_sums_slow<BATES>(C, p, tn, h * wj, g);
 #pragma unroll
                         for (int k = 0; k < DIM; ++k) sum[k] += g[k];
                     }
@@ -201,10 +203,14 @@ __global__ void __launch_bounds__(128, BATES ? OPE_GRAD_MINB_BATES : OPE_GRAD_MI
             if (finite || !fast) break;  // else each node again, dropping the terms that are not finite
         }
         if (lane == 0) {
-            heston_chain(G, acc);
-            double* out = B.part + w * DIM;
+            double pe[8];
 #pragma unroll
-            for (int k = 0; k < DIM; ++k) out[k] = acc[k];
+            for (int i = 0; i < DIM; ++i) pe[i] = __ldcg(p + i);  // again: nothing of it is kept over the nodes
+            heston_chain(make_grad_params(pe, BATES), acc);
+            double* out = B.part + w * DIM;
+            // not finite here: 0 (every node dropped) times such a coefficient
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) out[k] = isfinite(acc[k]) ? acc[k] : 0.0;
         }
     }
 }

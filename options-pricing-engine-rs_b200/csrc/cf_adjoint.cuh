@@ -203,13 +203,25 @@ __device__ __forceinline__ void jump_partials(const CfConsts& C, const GradParam
     out[2] = (n.jump * phi2 + iphi * (1.0 + C.comp)) * (-C.lt * G.sigma_j);
 }
 
+// The parameter derivatives of an integral from its sums of the five Heston
+// quantities (linear, see the top); the jump derivatives are sums already.
+__device__ __forceinline__ void heston_chain(const GradParams& G, double* a) {
+    const double d0 = a[0], ch = a[1], y = a[2], ys = a[3], xw = a[4];
+    a[0] = d0;
+    a[1] = fma(G.tis2, ch, y);
+    a[2] = G.kis2 * ch;
+    a[3] = fma(G.rho, ys, fma(G.sigma, xw, -G.sk * ch));
+    a[4] = G.sigma * ys;
+}
+
 // One node's terms hw Im(W X) of the derivative sums, X the five Heston
 // quantities, then the jump derivatives.  A node whose value or a derivative
 // is not finite contributes zero, as in gk_integrate_dual (ad.rs:679-682).
 // FAST adds to acc and returns false (nothing added) where its functions do
 // not apply; it tests the value only, so that a derivative that is not finite
 // shows in acc and the caller takes its nodes again one by one, not FAST
-// (which writes the terms to acc).
+// (which writes the terms to acc, after testing the parameter derivatives that
+// they make).
 template <bool BATES, bool FAST>
 __device__ __forceinline__ bool node_sums(const CfConsts& C, const GradParams& G, double tn, double hw, double* acc) {
     constexpr int DIM = BATES ? 8 : 5;
@@ -227,34 +239,27 @@ __device__ __forceinline__ bool node_sums(const CfConsts& C, const GradParams& G
             for (int k = 0; k < DIM; ++k) acc[k] = fma(W.re, x[k].im, fma(W.im, x[k].re, acc[k]));
         }
     } else {
-        double g[8];
+        double g[8], d[8];
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) {
-            g[k] = hw * (n.W * x[k]).im;
-            ok = ok && isfinite(g[k]);
-        }
+        for (int k = 0; k < DIM; ++k) d[k] = g[k] = hw * (n.W * x[k]).im;
+        heston_chain(G, d);
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) ok = ok && isfinite(d[k]);
 #pragma unroll
         for (int k = 0; k < DIM; ++k) acc[k] = ok ? g[k] : 0.0;
     }
     return true;
 }
 
-// Its terms in g[0..DIM), by CUDA's functions.
+// Its terms in g[0..DIM), by CUDA's functions; p: the parameter set (read anew,
+// so that the caller's copy of the chain need not lie in memory for this call).
 template <bool BATES>
-static __device__ __noinline__ void node_sums_slow(const CfConsts& C, const GradParams& G, double tn, double hw,
+static __device__ __noinline__ void node_sums_slow(const CfConsts& C, const double* p, double tn, double hw,
                                                    double* g) {
-    node_sums<BATES, false>(C, G, tn, hw, g);
-}
-
-// The parameter derivatives of an integral from its sums of the five Heston
-// quantities (linear, see the top); the jump derivatives are sums already.
-__device__ __forceinline__ void heston_chain(const GradParams& G, double* a) {
-    const double d0 = a[0], ch = a[1], y = a[2], ys = a[3], xw = a[4];
-    a[0] = d0;
-    a[1] = fma(G.tis2, ch, y);
-    a[2] = G.kis2 * ch;
-    a[3] = fma(G.rho, ys, fma(G.sigma, xw, -G.sk * ch));
-    a[4] = G.sigma * ys;
+    double pl[8];
+#pragma unroll
+    for (int i = 0; i < (BATES ? 8 : 5); ++i) pl[i] = __ldg(p + i);
+    node_sums<BATES, false>(C, make_grad_params(pl, BATES), tn, hw, g);
 }
 
 // The exponent's derivatives for the analytic Greeks (x = ln(S/K) and r enter
