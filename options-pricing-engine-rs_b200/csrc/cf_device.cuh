@@ -759,7 +759,8 @@ __device__ __forceinline__ double node_u_of(double tn) {
 
 // FAST: branch-free, with the functions above; returns whether they applied: u
 // in the integral's range (CfConsts::u_span) and Z below 2^43, its real part
-// below 700 (so that the value is finite).  Not FAST: CUDA's functions and the
+// below 600: with 1e-12 <= u < 1e30 the factor 1/((1 - t) t) is below 2e30, so
+// that W stays below 1e291 and the sums over 200 panels are finite.  Not FAST: CUDA's functions and the
 // square root's other branch.
 //
 // What bounds it: register-file reads and issue slots (an FMA of three
@@ -846,7 +847,7 @@ __device__ __forceinline__ bool node_eval(const CfConsts& C, double tn, NodeCf& 
     n.w = __dmul_rn(FAST ? exp_node(zre) : exp(zre), itt);
     if (!FAST) return true;
     const int hz = __double2hiint(zre);
-    return (unsigned)__double2hiint(u) - kULow < C.u_span && hz < 0x4085E000 && (unsigned)hz < 0xC2A00000u &&
+    return (unsigned)__double2hiint(u) - kULow < C.u_span && hz < 0x4082C000 && (unsigned)hz < 0xC2A00000u &&
            node_range(zim) < 2u * 0x42A00000u;
 }
 
