@@ -343,8 +343,9 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
             }
         }
         __syncwarp();  // every lane has read entry w before it is overwritten
-        // swap_remove: the last entry takes the bisected one's slot
-        if (lane < 4) *reinterpret_cast<unsigned long long*>(list + (R.copy_at + w * R.copy_by)) = word;
+        // swap_remove: the last entry takes the bisected one's slot (its own: stays,
+        // as the left child, written by one lane above, is the next into it)
+        if (lane < 4 && w != last) *reinterpret_cast<unsigned long long*>(list + (R.copy_at + w * R.copy_by)) = word;
         if (CACHED && lane == 0) rc->slot[w] = (uint8_t)moved;
     }
     *nbis = len - 1;
