@@ -212,12 +212,6 @@ constexpr size_t kPipelineMin = 262144;
 // pageable copy each way around the launch: a small call's time is mostly
 // these fixed costs.
 constexpr size_t kStagedMax = 16384;
-// Other small inputs and results go through the pinned buffer up to this many
-// bytes, as one copy each way.  Host memcpy + copy from pinned against a
-// pageable copy, us, host to device / back: 57 kB 12 / 13 against 46 / 18,
-// 430 kB 26 / 27 against 36 / 44, 1.1 MB 57 / 58 against 74 / 98, 2.0 MB 158 /
-// 157 against 112 / 156.
-constexpr size_t kStagedBytes = 3 << 19;
 
 // The staged small-call setup: contracts copied into the pinned buffer
 // (*k_con points at them); *h_out is the pinned slot for the prices (NULL

@@ -60,6 +60,13 @@ int ensure_device();                               // OPE_OK or OPE_ERR_NO_DEVIC
 // `st`), so it never waits for, or stalls, work on other streams.
 int ensure_workspace(size_t bytes, void** out, cudaStream_t st);
 int ensure_pinned(size_t bytes, void** out);       // grows the pinned staging buffer
+// Small inputs and results of a host call go through the pinned buffer up to
+// this many bytes, as one copy each way (beyond, the page-locked memory that a
+// thread keeps would grow with its calls).  Host memcpy + copy from pinned
+// against a pageable copy, us, host to device / back: 57 kB 12 / 13 against 46 /
+// 18, 430 kB 26 / 27 against 36 / 44, 1.1 MB 57 / 58 against 74 / 98, 2.0 MB
+// 158 / 157 against 112 / 156.
+constexpr size_t kStagedBytes = 3 << 19;
 // Resident blocks per SM of `kernel` (threads per block, dynamic shared
 // memory) on the current device, with its dynamic-shared-memory attribute
 // set; queried once per kernel and device, then cached.
