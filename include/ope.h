@@ -375,13 +375,16 @@ int ope_price_surfaces_noalloc(int32_t model, const ope_contract* d_contracts, s
  * ope_autotune measures every candidate shape (1, 2 or 4 warps x order x
  * occupancy 1 or 1/2) on seeded synthetic batches of each size class (at the
  * class's geometric interior) on the calling thread's device, keeps per class
- * the fastest shape if it beats the default (4, input order, 1) by more than
- * 3 %, installs the table for that device and model in this process, and
- * writes the OPE_TUNE_CLASSES entries to out_entries (may be NULL).  Takes
+ * the fastest shape if it beats the automatic launch by more than 3 %, installs
+ * the table for that device and model in this process, and writes the
+ * OPE_TUNE_CLASSES entries to out_entries (may be NULL).  The automatic launch,
+ * which the default shape (4, input order, 1, per_unit 0) stands for in a
+ * table, chooses order and resident warps by the size and depth of the call;
+ * an entry that differs from it in any field is taken as it is.  Tuning takes
  * about 10 s (about 1 s with OPE_TUNE_QUICK).  Plain pricing calls (ope_batch_*,
  * ope_price_surfaces, Greeks, the server's reprices) then launch with their
- * class's shape; calibration passes keep the default shape.
- * ope_set_autotune(0) returns every call to the default shape (1: the tuned
+ * class's shape; calibration passes ignore the table.
+ * ope_set_autotune(0) returns every call to the automatic launch (1: the tuned
  * tables again); ope_get_tune_table reads the current device's table
  * (*out_tuned = 0: not tuned, the default entries); ope_set_tune_table
  * installs one. */
@@ -402,7 +405,7 @@ typedef struct {
 typedef struct {
     uint64_t max_contracts;  /* the class: calls of at most this many contracts (the last: all larger) */
     ope_launch_shape shape;  /* the shape calls of this class use */
-    double ms_default;       /* measured kernel time of the default shape on the class's batch */
+    double ms_default;       /* measured kernel time of the automatic launch on the class's batch */
     double ms_tuned;         /* measured kernel time of `shape` (ms_default when it is the default) */
 } ope_tune_entry;
 #define OPE_TUNE_CLASSES 16  /* calls of up to 64, 128, 256, ..., 2^20 contracts, and larger */

@@ -160,8 +160,8 @@ struct LaunchShape {
     // its contracts on the device and takes the run kernel when its runs
     // average 4 contracts or more
     int per_unit = 0;
-    // not from a tuned table: queue order and resident warps go by the call
-    // (pricing.cu: order_by_size, k_order_scatter)
+    // the automatic launch (no tuned table, or its default shape): queue order and
+    // resident warps go by the call (pricing.cu: order_by_size, k_order_scatter)
     bool by_size = true;
 };
 // Bytes of the run cache for the current device (every warp the run

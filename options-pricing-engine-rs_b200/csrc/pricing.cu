@@ -807,7 +807,7 @@ int launch_price_persistent(int model, const ope_contract* con, size_t n, const 
     LaunchShape sh;
     const bool can_order = s.order && n <= 0xffffffffull;
     if (!sink && !surf_mask) sh = shape ? *shape : price_shape(model, n);
-    const bool by_size = sh.by_size && !shape && !surf_mask && can_order && order_by_size(n, n_surf, param_idx);
+    const bool by_size = sh.by_size && !surf_mask && can_order && order_by_size(n, n_surf, param_idx);
     if (by_size) sh.deepest_first = 1;
     if (!can_order) sh.deepest_first = 0;
     // contracts per unit: fixed (2..32), automatic (0: probe for runs where

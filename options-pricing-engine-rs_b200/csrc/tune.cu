@@ -8,8 +8,9 @@
 // device in use, every candidate shape on seeded synthetic batches of each
 // size class (powers of two from 64 to 2^20 contracts, and larger;
 // benchmark-configuration parameter ranges)
-// and keeps, per class, the fastest shape when it beats the default by more
-// than 3 % (else the default):
+// and keeps, per class, the fastest shape when it beats the automatic launch
+// (pricing.cu: order and resident warps by the size and depth of the call) by
+// more than 3 %, else the default shape, which stands for the automatic launch:
 //   * warps per block: 1, 2 or 4 (each warp one integral), i.e. how finely
 //     a small call's units spread over the SMs;
 //   * queue order: input order, or deepest-first by |ln(K/S)| / sqrt(v0 T);
@@ -17,7 +18,7 @@
 //     SM sub-partition run each chain faster).
 // The panel list keeps the reference's 200-panel capacity (a smaller one
 // would change results; shared memory does not limit occupancy at the
-// 64-register budget), and each integral keeps one warp (several warps per
+// 72-register budget), and each integral keeps one warp (several warps per
 // integral were measured slower).  The table lives per device in this
 // process; ope_autotune fills it, ope_set_autotune switches it on or off.
 #include <cuda_runtime.h>
@@ -129,6 +130,12 @@ ope_tune_entry default_entry(int cls) {
     return e;
 }
 
+bool is_default(const ope_launch_shape& s) {
+    const ope_launch_shape d = default_entry(0).shape;
+    return s.warps_per_block == d.warps_per_block && s.deepest_first == d.deepest_first &&
+           s.occupancy == d.occupancy && s.per_unit == d.per_unit;
+}
+
 struct DevBatch {
     ope_contract* con = nullptr;
     int64_t* off = nullptr;
@@ -170,7 +177,8 @@ LaunchShape price_shape(int model, size_t n) {
     const auto it = g_tables.find(dev);
     if (it == g_tables.end() || !it->second.tuned[m]) return sh;
     const ope_tune_entry& e = it->second.e[m][class_of(n)];
-    sh.by_size = false;
+    // the default shape is the automatic launch; any other is taken as it is
+    sh.by_size = is_default(e.shape);
     sh.warps = e.shape.warps_per_block;
     sh.deepest_first = e.shape.deepest_first;
     sh.occupancy = e.shape.occupancy;
@@ -238,7 +246,7 @@ int ope_autotune(int32_t model, uint32_t flags, ope_tune_entry* out_entries) {
                                  "cudaMemcpyAsync")) != OPE_OK)
                 break;
             const int warm = n >= 185364 ? 1 : 3, reps = n >= 185364 ? 3 : (n >= 11585 ? 5 : 9);
-            LaunchShape def;
+            LaunchShape def;  // the automatic launch, as an untuned call takes it
             double t_def = 0.0;
             if ((rc = time_shape(model, B, n, ns, 1e-10, def, warm, reps, c.stream, e0, e1, &t_def)) != OPE_OK) break;
             LaunchShape best = def;
@@ -246,8 +254,9 @@ int ope_autotune(int32_t model, uint32_t flags, ope_tune_entry* out_entries) {
             for (int w : {1, 2, 4})
                 for (int df : {0, 1})
                     for (double occ : {1.0, 0.5}) {
-                        const LaunchShape sh{w, df, occ};
-                        if (w == 4 && df == 0 && occ == 1.0) continue;
+                        LaunchShape sh{w, df, occ};
+                        sh.by_size = false;
+                        if (w == 4 && df == 0 && occ == 1.0) continue;  // the automatic launch's shape
                         double t = 0.0;
                         if ((rc = time_shape(model, B, n, ns, 1e-10, sh, warm, reps, c.stream, e0, e1, &t)) != OPE_OK)
                             break;
