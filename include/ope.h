@@ -442,21 +442,44 @@ int ope_trace_integral(int32_t model, const ope_contract* contract, const void* 
                        double* out_steps, int32_t max_steps, int32_t* out_n_steps, double* out_integral);
 
 /* No reference twin (numerics self-check): the worst error, in ulps, of the
- * kernels' Newton-refined reciprocal and square root against IEEE 1/x and
+ * kernels' refined reciprocal and square root against IEEE 1/x and
  * sqrt over 2^20 inputs spanning 1e-300 .. 1e300. */
 int ope_selftest_math(uint64_t* max_ulp_rcp, uint64_t* max_ulp_sqrt);
 
 /* No reference twin (numerics self-check): the worst difference, in ulps, of
- * the node evaluation's own branch-free atan2 (used for arg A of the Albrecher
- * CF, heston.rs:120) from CUDA's atan2 over 2^24 argument pairs with
- * magnitudes 2^-60 .. 2^60 and ratios 2^-45 .. 2^45. */
+ * the library's own branch-free atan2 from CUDA's atan2 over 2^24 argument
+ * pairs with magnitudes 2^-60 .. 2^60 and ratios 2^-45 .. 2^45.  (The node
+ * evaluation's argument is OPE_NODE_ARG below.) */
 int ope_selftest_atan2(uint64_t* max_ulp);
 
 /* No reference twin (numerics self-check): the worst difference, in ulps, of
- * the node evaluation's own log (used for log|A| of the Albrecher CF,
- * heston.rs:120) from CUDA's log over 2^24 arguments from 2^-1000 to 2^1000
- * and around 1. */
+ * the library's own log from CUDA's log over 2^24 arguments from 2^-1000 to
+ * 2^1000 and around 1.  (The node evaluation's logarithm is
+ * OPE_NODE_LOG_RATIO below.) */
 int ope_selftest_log(uint64_t* max_ulp);
+
+/* No reference twin (numerics self-check): one of the functions the node
+ * evaluation of the pricing and gradient kernels is made of, on the device, at
+ * n pairs of host arguments (a, b) (n <= 2^26; b is read but unused where
+ * it is not named):
+ *   OPE_NODE_EXP        e^a                 OPE_NODE_COS, _SIN      cos a, sin a
+ *   OPE_NODE_COS_SUM,
+ *   OPE_NODE_SIN_SUM    cos, sin of a + b   OPE_NODE_SIN_VALUE      sin(a + b)
+ *   OPE_NODE_LOG_RATIO  log(a / b)          OPE_NODE_LOG_RCP        1 / a, from the same call
+ *   OPE_NODE_ARG        arg(b + i a)
+ * They apply to |a|, |b| < 2^44 for the phases and, for the logarithm, to
+ * positive normal numbers whose product is normal; e^a is held at about 1e-308
+ * below a = -708 and may be not finite from 709.77 on. */
+#define OPE_NODE_EXP 0
+#define OPE_NODE_COS 1
+#define OPE_NODE_SIN 2
+#define OPE_NODE_COS_SUM 3
+#define OPE_NODE_SIN_SUM 4
+#define OPE_NODE_SIN_VALUE 5
+#define OPE_NODE_LOG_RATIO 6
+#define OPE_NODE_LOG_RCP 7
+#define OPE_NODE_ARG 8
+int ope_selftest_node_function(int32_t which, const double* a, const double* b, size_t n, double* out);
 
 /* No reference twin (numerics self-check of heston.rs:223, u = (1 - t)/t):
  * the number of 2^24 node positions t, uniform in (0, 1) and log-uniform down

@@ -781,6 +781,16 @@ int ope_selftest_node_u(uint64_t* mismatches) {
     return selftest_node_u(mismatches);
 }
 
+int ope_selftest_node_function(int32_t which, const double* a, const double* b, size_t n, double* out) {
+    OPE_RANGE("ope.selftest_node_function");
+    if (which < OPE_NODE_EXP || which > OPE_NODE_ARG) return set_error(OPE_ERR_INVALID_ARG, "no such function");
+    if (n == 0) return OPE_OK;
+    if (!a || !b || !out) return set_error(OPE_ERR_INVALID_ARG, "NULL argument");
+    if (n > ((size_t)1 << 26)) return set_error(OPE_ERR_INVALID_ARG, "n above 2^26");
+    OPE_TRY(ensure_device());
+    return selftest_node_function(which, a, b, n, out);
+}
+
 int ope_selftest_log_cr(const double* args, size_t n, double* out_log_cr, double* out_log_cuda) {
     OPE_RANGE("ope.selftest_log_cr");
     if (n == 0) return OPE_OK;

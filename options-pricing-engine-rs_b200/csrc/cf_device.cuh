@@ -66,9 +66,8 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
     return fma(y, fma(1.5 * e, e, e), y);
 }
 
-// arg(A) of the node evaluation's Log A: atan2(y, x), branch-free, written
-// for this use (CUDA's atan2 was the costliest call of a node: replacing it
-// cut the Bates batch by 4 %).  Method (the classical argument reduction of
+// atan2(y, x), branch-free (the node evaluation's own argument is arg_node; this
+// one is what ope_selftest_atan2 compares).  Method (the classical argument reduction of
 // Cody and Waite's elementary-function manual): octant symmetry reduces it
 // to atan(q), q = min(|x|,|y|)/max(|x|,|y|) in [0, 1]; above tan(pi/8),
 // atan(q) = pi/4 + atan((q - 1)/(q + 1)); on |t| <= tan(pi/8),
@@ -76,10 +75,8 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
 // of node_math_coeffs.py (5e-18 relative).  With q = mn/mx the reduced quotient
 // is (mn - mx)/(mn + mx), so one rcp_nr serves either case.  At most
 // 4 ulp from CUDA's atan2 over finite arguments whose larger magnitude is at
-// least 2^-1022 (ope_selftest_atan2); outside that (a NaN or infinite
-// argument, or both below 2^-1022) it returns NaN.  In the node evaluation
-// those cases come only from an A that is 0, infinite or NaN, where log|A| is
-// not finite and the node's value is 0 with either function.
+// least 2^-1022; outside that (a NaN or infinite argument, or both below
+// 2^-1022) it returns NaN.
 __device__ __forceinline__ double atan2_node(double y, double x) {
     const double ax = fabs(x), ay = fabs(y);
     const bool swap = ay > ax;
@@ -222,15 +219,15 @@ __device__ __forceinline__ double arg_node(double y, double x) {
     return __dadd_rn(__ldg(&e->k), fma(__dmul_rn(t, s), p, t));
 }
 
-// log|A|^2 of the node evaluation's Log A: log(v), written for this use
-// (2.4 % off the Bates batch against CUDA's log).  Method (the atanh form of
+// log(v) (the node evaluation's own logarithm is log_ratio, made the same way;
+// this one is what ope_selftest_log compares).  Method (the atanh form of
 // the logarithm of Cody and Waite's manual): v = 2^k m with m in
 // [sqrt(1/2), sqrt 2), read off the IEEE exponent and mantissa bits;
 // log v = k ln 2 + 2 atanh(s), s = (m - 1)/(m + 1) (m - 1 is exact, the
 // quotient uses rcp_nr), 2 atanh(s) = 2 s + s w R(w), w = s^2, with the
 // degree-6 Chebyshev interpolant R of node_math_coeffs.py (4.5e-18 relative),
 // and k ln 2 added through two FMAs with ln 2 split into a double and its
-// remainder.  At most 2 ulp from CUDA's log (ope_selftest_log).  Arguments
+// remainder.  At most 2 ulp from CUDA's log.  Arguments
 // outside the normal range (0, subnormal, infinite, NaN) take CUDA's log.
 __device__ __forceinline__ double log_node(double v) {
     const int hi = __double2hiint(v), lo = __double2loint(v);
@@ -351,8 +348,8 @@ __device__ __forceinline__ unsigned node_range(double x) { return 2u * (unsigned
 // (9e-18 absolute, node_math_coeffs.py), ln2/64 split into 21 bits and the
 // rest.  x is held between -708 and 710 by its high word (as unsigned a more
 // negative double is larger, as signed a negative one is negative), so that k
-// fits the low word: below, some 1e-308 instead of 0, above 709.8 infinity or
-// NaN; a NaN may come out as either end, its callers test x.  In place of CUDA's
+// fits the low word: below, some 1e-308 instead of 0, above 709.777 (k = 2^16, past
+// 2^1023) infinity or NaN; a NaN may come out as either end, its callers test x.  In place of CUDA's
 // exp on the 262k-contract Bates batch: 11.05 -> 10.61 ms (after cis_node and
 // sin_node); a degree-11 polynomial without the table: 10.96 ms.
 __device__ __forceinline__ double exp_node(double x) {
@@ -548,22 +545,6 @@ __device__ __forceinline__ Cx fast_csqrt(double a, double b) {
     double w = sqrt(0.5 * (r + fabs(a)));
     double q = (w > 0.0) ? (0.5 * b) / w : b;
     return (a >= 0.0) ? Cx{w, q} : Cx{fabs(q), copysign(w, b)};
-}
-
-// d = fast_csqrt(z) of the node evaluations (heston.rs:155-175), branch-free
-// and without hypot, a division or an IEEE square root: |z| and
-// w = sqrt((|zr| + |z|)/2) through refined reciprocal square roots, the other
-// component zi / (2 w).  z = 0 gives d = 0 as the reference's b == 0 branch
-// does.
-__device__ __forceinline__ void csqrt_node(double zr, double zi, double& dre, double& dim) {
-    const double zz = fma(zr, zr, zi * zi);
-    const double r = (zz > 0.0) ? zz * rsqrt_nr(zz) : zz;  // |z| (zz = 0 stays 0)
-    const double s2 = 0.5 * (r + fabs(zr));
-    const double iw = rsqrt_nr(s2);
-    const double w = (s2 > 0.0) ? s2 * iw : 0.0;
-    const double q = (s2 > 0.0) ? (0.5 * zi) * iw : zi;
-    dre = (zr >= 0.0) ? w : fabs(q);
-    dim = (zr >= 0.0) ? q : copysign(w, zi);
 }
 
 // Per-integral constants (everything that does not depend on the node),

@@ -1,5 +1,5 @@
-"""Coefficients of the node evaluation's own atan2 and log (cf_device.cuh:
-atan2_node, log_node), computed in 60-digit arithmetic (mpmath).
+"""Coefficients of cf_device.cuh's own functions, computed in 60-digit arithmetic
+(mpmath): first those of atan2_node and log_node, which its self-tests alone use.
 
 atan2_node reduces atan2(y, x) to atan(t) with |t| <= tan(pi/8): first to
 q = min(|x|,|y|) / max(|x|,|y|) in [0, 1] (octant symmetry), then, for
@@ -14,7 +14,7 @@ log v = k ln 2 + 2 atanh(s), s = (m - 1)/(m + 1), |s| <= 3 - 2 sqrt 2, and
 interpolates (2 atanh(s) - 2 s)/(s w) at the 7 Chebyshev nodes of
 [0, (3 - 2 sqrt 2)^2]: 4.5e-18 relative error on log m.
 
-The functions below are the node evaluation's own (log_ratio, exp_node,
+The node evaluation is made of the functions below (log_ratio, exp_node,
 cis_node, sin_node, arg_node).  Their leading coefficients have a zero low word
 (at most 21 significant bits): an FP64 instruction takes such a constant as an
 immediate, where a full double costs a load and a third 64-bit register operand
@@ -30,9 +30,9 @@ so the rounding costs nothing as long as the result stays near 1e-17:
   arg_node:  atan t = t + t^3 P(t^2), |t| <= 0.1125, degree 5, 3 short.
 
 All are far below the 1.1e-16 rounding unit; the evaluation in double
-precision then adds a few ulps (checked against CUDA's functions on the
-device by ope_selftest_atan2 / ope_selftest_log and in numpy by
-tests/test_node_math_cpu.py).
+precision then adds a few ulps (checked on the device through
+ope_selftest_atan2, ope_selftest_log and ope_selftest_node_function, and in
+numpy by tests/test_node_math_cpu.py and tests/test_node_functions_cpu.py).
 
 Run: python node_math_coeffs.py  (prints the coefficients, highest degree
 first, as they appear in cf_device.cuh, and the approximation errors).

@@ -103,7 +103,45 @@ __global__ void k_eval_log_cr(const double* v, long long n, double* out_cr, doub
     out_cuda[i] = log(v[i]);
 }
 
+// The node evaluation's functions on given arguments (ope.h:
+// ope_selftest_node_function).
+__global__ void k_eval_node_function(int which, const double* a, const double* b, long long n, double* out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double x = a[i], y = b[i];
+    double re = 0.0, im = 0.0;
+    switch (which) {
+        case OPE_NODE_EXP: out[i] = exp_node(x); return;
+        case OPE_NODE_COS:
+        case OPE_NODE_SIN: cis_node(x, re, im); out[i] = which == OPE_NODE_COS ? re : im; return;
+        case OPE_NODE_COS_SUM:
+        case OPE_NODE_SIN_SUM: cis_node(x, y, re, im); out[i] = which == OPE_NODE_COS_SUM ? re : im; return;
+        case OPE_NODE_SIN_VALUE: out[i] = sin_node(x, y, 1.0); return;
+        case OPE_NODE_LOG_RATIO: out[i] = log_ratio(x, y, re); return;
+        case OPE_NODE_LOG_RCP: log_ratio(x, y, re); out[i] = re; return;
+        default: out[i] = arg_node(x, y); return;  // OPE_NODE_ARG
+    }
+}
+
 }  // namespace
+
+int selftest_node_function(int which, const double* a, const double* b, size_t n, double* out) {
+    ThreadCtx& c = tctx();
+    const size_t bytes = align_up(n * sizeof(double), 256);
+    void* ws;
+    OPE_TRY(ensure_workspace(3 * bytes, &ws, c.stream));
+    double* d_a = static_cast<double*>(ws);
+    double* d_b = reinterpret_cast<double*>(static_cast<char*>(ws) + bytes);
+    double* d_o = reinterpret_cast<double*>(static_cast<char*>(ws) + 2 * bytes);
+    OPE_CHECK(cudaMemcpyAsync(d_a, a, n * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    OPE_CHECK(cudaMemcpyAsync(d_b, b, n * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    k_eval_node_function<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(which, d_a, d_b, (long long)n, d_o);
+    OPE_CHECK(cudaGetLastError());
+    c.launches += 1;
+    OPE_CHECK(cudaMemcpyAsync(out, d_o, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    OPE_CHECK(cudaStreamSynchronize(c.stream));
+    return OPE_OK;
+}
 
 int selftest_log_cr(const double* v, size_t n, double* out_cr, double* out_cuda) {
     ThreadCtx& c = tctx();

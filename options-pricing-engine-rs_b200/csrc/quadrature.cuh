@@ -72,7 +72,6 @@ struct alignas(16) PanelStore {
 // Per-lane quadrature constants, loaded once per warp.
 struct LaneRule {
     double x, wk, wg;
-    bool node;  // lane holds a Kronrod node (lane % 16 < 15)
     int half;   // 0 = left child, 1 = right child
     // reduce-scatter weights: of the K15 and G7 weights of this lane's node,
     // the one whose product the lane keeps (G7 if lane bit 3 is set) and the
@@ -89,7 +88,6 @@ __device__ __forceinline__ LaneRule lane_rule(int lane) {
     R.x = c_gk_x[j];
     R.wk = c_gk_wk[j];
     R.wg = c_gk_wg[j];
-    R.node = j < 15;
     R.half = lane >> 4;
     R.wkeep = (lane & 8) ? R.wg : R.wk;
     R.wsend = (lane & 8) ? R.wk : R.wg;
