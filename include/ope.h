@@ -397,8 +397,9 @@ typedef struct {
                               * set with the same expiry and rate (the strikes of one expiry of a surface
                               * laid out expiry by expiry) evaluates the characteristic function once per
                               * panel for the whole run (4 warps, input order).  0 (the default):
-                              * automatic -- a large call (151,552 contracts or more on 148 SMs) counts its runs on the
-                              * device and takes blocks of 16 when they average 4 contracts or more.
+                              * automatic -- a large call (576 contracts per SM or more: 85,248 on 148)
+                              * counts its runs on the device and takes blocks of 4, 8 or 16 when they
+                              * average as many contracts and leave every warp its units.
                               * Prices are bit-identical in every mode. */
     int32_t reserved;        /* 0 */
 } ope_launch_shape;
@@ -410,7 +411,7 @@ typedef struct {
 } ope_tune_entry;
 #define OPE_TUNE_CLASSES 16  /* calls of up to 64, 128, 256, ..., 2^20 contracts, and larger */
 #define OPE_TUNE_QUICK 1u    /* ope_autotune flag: measure the classes up to 2^17 contracts only (the
-                              * larger ones keep the default shape) */
+                              * larger ones keep the automatic launch) */
 int ope_autotune(int32_t model, uint32_t flags, ope_tune_entry* out_entries);
 /* Contracts per unit that this thread's last plain pricing call launched
  * with (1: one per unit; for an automatic launch, the run probe's choice --

@@ -173,7 +173,7 @@ constexpr int kTuneClasses = 16;  // OPE_TUNE_CLASSES
 extern const uint64_t kTuneClassMax[kTuneClasses];
 // The shape a plain pricing launch of n contracts of `model` uses on the
 // current device: the tuned table's entry for n's class when this device has
-// been tuned and tuning is enabled, else the default shape.
+// been tuned and tuning is enabled, else the automatic launch.
 LaunchShape price_shape(int model, size_t n);
 
 // Device launchers (stream-ordered; all pointers are device pointers).

@@ -45,7 +45,7 @@ constexpr int kOrderBuckets = 64;
 constexpr int kSmSlots = 256;  // resident-block counters, by %smid (in the order's bucket array)
 constexpr size_t kHistBytes = 2 * kOrderBuckets * sizeof(unsigned int);
 // Run cache entries per warp (panels of one run), and warps per SM it is
-// sized for (the 64-register budget holds at most 32).
+// sized for (all that OPE_RUNS_MINB's 80 registers hold).
 #ifndef OPE_RUN_CACHE_ENTRIES
 #define OPE_RUN_CACHE_ENTRIES kRunEntries
 #endif
@@ -375,8 +375,8 @@ __global__ void __launch_bounds__(64, 8)
 // instead of once per panel and strike.  A run never reaches across blocks.
 // Prices are bit-identical to k_price_persistent's.
 //
-// What bounds it: issue slots (77 % used), most of them the step's bookkeeping
-// (350 instructions per step, of which 100 FP64).  Without a per-run switch, with
+// What bounds it: issue slots (73 % used), most of them the step's bookkeeping
+// (305 instructions per step, of which 77 FP64).  Without a per-run switch, with
 // a node's (W, A) as one 16-byte word, a sentinel entry in place of branches and
 // the node evaluation inline again (out of line, a miss saved and restored the
 // loop's registers through local memory): 24.7 -> 23.3 ms on 1.46M Heston grid

@@ -203,7 +203,7 @@ struct NoTrace {
 // bisection go through ONE call site of the integrand, so the (large) inlined
 // node evaluation exists once in the instruction stream.
 //
-// CACHED: with the run cache `rc` (which may be off for this integral): each
+// CACHED: with the run cache `rc`: each
 // step first looks its panel(s) up in the tree (a hit: both children, or the
 // root, already evaluated) and otherwise evaluates node_cf and, while the
 // tree has room and the bisected panel is in it, stores the children.
@@ -223,7 +223,7 @@ __device__ __forceinline__ double gk_integrate_warp(const CfConsts& C, double to
     for (int j = 0; j < (kMaxPanels + 31) / 32; ++j)
         if (lane + 32 * j < kMaxPanels) L.ekey[lane + 32 * j] = 0ull;
     __syncwarp();
-    // cache mode of the step (warp-uniform): hit = read entries el_/er_,
+    // cache mode of the step (warp-uniform): hit = read entries el_ and el_ + 1,
     // put = evaluate and store into them; neither = evaluate uncached.  The
     // first step's panel [0, 1] is entry 0.
     bool hit = false, put = false;

@@ -510,7 +510,7 @@ def autotune(model: int, quick: bool = False) -> list[dict]:
 
 
 def set_autotune(enabled: bool) -> None:
-    """Use the tuned tables (True) or the default launch shape (False)."""
+    """Use the tuned tables (True) or the automatic launch for every call (False)."""
     check(load().ope_set_autotune(1 if enabled else 0))
 
 
